@@ -28,6 +28,7 @@
 #include "xr_kernel.cuh"
 #include "oft3_kernel.cuh"
 #include "oft4_kernel.cuh"
+#include "small_kernel.cuh"
 
 namespace {
 
@@ -50,7 +51,7 @@ int fail(int code, const char* fmt, ...) {
 // library choose".  The B200_* environment variables of the same meaning are read ONCE, at the first use
 // of any option in the process, as initial values; after that only b200_set_option changes them, so
 // nothing on the launch path reads the environment.
-enum OptionId { kOptOftRoute, kOptRaster, kOptTileSync, kOptL2Hints, kOptGemmTileSync, kOptGemmL2Hints, kOptGemmSplit, kOptMaps3d, kOptRingBands, kOptPrefetch, kOptRotPairs, kOptCount };
+enum OptionId { kOptOftRoute, kOptRaster, kOptTileSync, kOptL2Hints, kOptGemmTileSync, kOptGemmL2Hints, kOptGemmSplit, kOptMaps3d, kOptRingBands, kOptPrefetch, kOptRotPairs, kOptSmallTiles, kOptSmallSplit, kOptPdl, kOptSmallStages, kOptCount };
 struct OptionDef { const char* name; const char* env; int initial; };
 constexpr OptionDef kOptionDefs[kOptCount] = {
     {"oft_route", "B200_OFT_PATH", 0},            // 0 choose, 1 X.R in tensor memory per tile, 2 two passes, 3 / 4 X.R shared through the L2 ring
@@ -64,6 +65,10 @@ constexpr OptionDef kOptionDefs[kOptCount] = {
     {"ring_bands", "B200_RING_BANDS", -1},        // bands of row blocks the X.R ring of route 3 holds (>= 2)
     {"prefetch", "B200_PREFETCH", -1},            // route 3: K steps by which W tiles are asked into L2 ahead of their load (0 off)
     {"rot_pairs", "B200_ROT_PAIRS", -1},          // route 4: SM pairs that only rotate (>= 1)
+    {"small_tiles", "B200_SMALL_TILES", -1},      // plain GEMM: 0 never the small-problem kernel, 1 always
+    {"small_split", "B200_SMALL_SPLIT", -1},      // small-problem kernel: pieces along K (1..8)
+    {"pdl", "B200_PDL", -1},                      // 0: no programmatic dependent launch
+    {"small_stages", "B200_SMALL_STAGES", -1},    // small-problem kernel: ring depth
 };
 std::atomic<int> g_opt[kOptCount];
 std::once_flag g_opt_once;
@@ -278,6 +283,116 @@ template <typename TIn, typename TOut, bool kNT, class P, int kBN>
 int launch_gemm_bn(int m, int n, int k, const void* A, int ldA, const void* B, int ldB, void* C, int ldC, void* stream_v,
                    int k2, const void* A2, int ldA2, const void* B2, int ldB2, float alpha, float beta);
 
+// ---- small problems: small_kernel ----------------------------------------------------------------------
+// Sizes that decide between the kernels (and how often K is cut) in the place of a call's own: an entry point that
+// computes one product in parts (row chunks, slabs of N) sets them to the whole product's, so that the parts have the
+// bits of a single call.
+thread_local int g_plan_m = 0, g_plan_n = 0;
+struct PlanAs {
+  PlanAs(int m, int n) { g_plan_m = m; g_plan_n = n; }
+  ~PlanAs() { g_plan_m = g_plan_n = 0; }
+};
+// Tiles of 128 x 128 of an m x n result.
+long long tiles_128(int m, int n) { return ((static_cast<long long>(m) + 127) / 128) * ((static_cast<long long>(n) + 127) / 128); }
+
+// Whether small_kernel takes an m x n result: as long as its 128 x 128 tiles do not outnumber the SMs.  Below the line
+// every one of 150 random shapes of the operator surface ran faster on it than on the pair kernels, by 1.1 to 6.7 times
+// (fixed cost per launch 5 us against 9 to 10 us, and 256 x 256 tiles leave most SMs idle: 8 x 4096 x 4096 OFT 35 -> 10
+// us, 640 x 1280 x 1024 TF32 29 -> 10 us); above it long K is the pair kernels' (2808 x 968 x 9590: 82 against 123 us).
+bool small_wins(int m, int n, const DeviceState* st) { return tiles_128(m, n) <= st->sm_count; }
+
+struct SmallPlan {
+  int tiles_m, tiles_n, n_tile, split, stages, xbufs, smem;
+};
+// Geometry for P [m][k], Q [n][k]; b > 0: Q is rotated by b x b blocks.
+template <class T>
+SmallPlan small_plan(int m, int n, int k, const DeviceState* st) {
+  constexpr int gran = T::kMn ? T::kChunk : 16, unit = T::kB == 128 ? 2 : 1;
+  constexpr int min_stages = T::kB == 128 ? 4 : 3;  // both steps of a 128 x 128 block, and the next block's behind them
+  constexpr int half_sm = 113 * 1024, whole_sm = 232448;
+  const int steps = (k + T::kBK * unit - 1) / (T::kBK * unit) * unit;
+  struct Ring { int n_tile, xbufs, stage, fixed, stages; bool two; };
+  auto ring = [&](int rows) {  // for a Q of this many rows
+    Ring r;
+    const int tiles = (rows + 127) / 128;
+    r.n_tile = ((rows + tiles - 1) / tiles + gran - 1) / gran * gran;
+    r.xbufs = T::kRot ? (r.n_tile <= 64 ? 3 : 2) : 0;
+    r.stage = r.n_tile * 128 + T::kRBytes + T::kPBytes;
+    r.fixed = 1024 + r.xbufs * r.n_tile * 128 + T::kTailBytes;
+    r.stages = (half_sm - r.fixed) / r.stage;
+    r.two = r.stages >= min_stages;  // two CTAs per SM
+    if (!r.two) r.stages = (whole_sm - r.fixed) / r.stage;
+    return r;
+  };
+  Ring r = ring(n);
+  // As many pieces along K as there is room for CTAs at once; at least four K steps each, and none below 16 steps (a
+  // K loop of 16 steps takes about 4 us, adding up the pieces 1.5).
+  const long long tiles = g_plan_m > 0 ? tiles_128(g_plan_m, g_plan_n) : tiles_128(m, n);
+  const long long slots = (ring(g_plan_m > 0 ? g_plan_m : n).two ? 2 : 1) * st->sm_count;
+  SmallPlan p;
+  p.split = 1;
+  if (steps >= 16)
+    while (p.split < 8 && tiles * (p.split + 1) <= slots && steps / (p.split + 1) >= 4) ++p.split;
+  if (opt(kOptSmallSplit) >= 1 && opt(kOptSmallSplit) <= 8) p.split = opt(kOptSmallSplit);
+  if (opt(kOptGemmSplit) == 0) p.split = 1;
+  if (p.split > steps / unit) p.split = steps / unit;
+  if (opt(kOptSmallStages) >= 2) r.stages = opt(kOptSmallStages);
+  if (r.stages > (whole_sm - r.fixed) / r.stage) r.stages = (whole_sm - r.fixed) / r.stage;
+  if (r.stages < min_stages) r.stages = min_stages;
+  if (r.stages > T::kMaxStages) r.stages = T::kMaxStages;
+  p.tiles_m = (m + 127) / 128;
+  p.tiles_n = (n + 127) / 128;
+  p.n_tile = r.n_tile;
+  p.xbufs = r.xbufs;
+  p.stages = r.stages;
+  p.smem = r.fixed + r.stages * r.stage;
+  if (p.smem < 78 * 1024) p.smem = 78 * 1024;  // at most two CTAs of an SM: their tensor memory (256 columns each) is all there is
+  return p;
+}
+
+template <class T>
+int launch_small(const SmallPlan& p, int m, int n, int k, const void* P, int ldP, const char* p_name, const void* Q, int ldQ, const char* q_name,
+                 const void* R, int ldR, int group_size, void* C, int ldC, float alpha, float beta, cudaStream_t stream, DeviceState* st) {
+  using TIn = typename T::TIn;
+  using TOut = typename T::TOut;
+  CUtensorMap mp, mq, mr;
+  int p3d = 0, q3d = 0;
+  if constexpr (!T::kMn) {
+    if (int rc = make_map(&mp, P, sizeof(TIn), k, m, ldP, T::kBK, T::kBM, p_name)) return rc;
+    if (int rc = make_map(&mq, Q, sizeof(TIn), k, n, ldQ, T::kBK, p.n_tile, q_name)) return rc;
+  } else {
+    const bool try3d = opt(kOptMaps3d) != 0;
+    if (try3d && make_map_chunks(&mp, P, sizeof(TIn), m, k, ldP, T::kChunk, T::kBK, T::kBM / T::kChunk, T::k32Atom) == B200_OK) p3d = 1;
+    else if (int rc = make_map(&mp, P, sizeof(TIn), m, k, ldP, T::kChunk, T::kBK, p_name, T::k32Atom)) return rc;
+    if (try3d && make_map_chunks(&mq, Q, sizeof(TIn), n, k, ldQ, T::kChunk, T::kBK, p.n_tile / T::kChunk, T::k32Atom) == B200_OK) q3d = 1;
+    else if (int rc = make_map(&mq, Q, sizeof(TIn), n, k, ldQ, T::kChunk, T::kBK, q_name, T::k32Atom)) return rc;
+  }
+  if constexpr (T::kRot) {
+    if (int rc = make_map(&mr, R, 2, k, static_cast<long long>(m / group_size) * T::kB, ldR, T::kBK, T::kB, "R")) return rc;
+  } else {
+    mr = mq;  // never read
+  }
+  const int vec = (reinterpret_cast<uintptr_t>(C) % (4 * sizeof(TOut))) == 0 && ldC % 4 == 0;
+  SmallArgs args{m, n, k, C, ldC, st->status, p.n_tile, p.tiles_n, p.split, p.stages, p.xbufs, group_size, p3d, q3d, vec, alpha, beta};
+  auto kernel = small_kernel<T>;
+  if (int rc = opt_in_smem(kernel, 232448)) return rc;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(p.tiles_m * p.tiles_n * p.split));
+  cfg.blockDim = dim3(T::kThreads);
+  cfg.dynamicSmemBytes = static_cast<size_t>(p.smem);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = opt(kOptPdl) != 0 ? 1 : 0;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = static_cast<unsigned>(p.split);
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = p.split > 1 ? 2 : 1;
+  CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, mp, mq, mr, args));
+  return B200_OK;
+}
+
 // (A pair kernel with half the N extent was tried for evening out the last wave of tiles and for small problems:
 // a half-width tile takes 0.8 of the time of a full one, M = N = K = 4096 TF32 0.286 ms against 0.203 ms, so it
 // never pays; the tiles of a short last wave are split along K instead, see below.)
@@ -309,6 +424,12 @@ int launch_gemm_bn(int m, int n, int k, const void* A, int ldA, const void* B, i
   }
   DeviceState* st;
   if (int rc = device_state(&st)) return rc;
+  if constexpr (kPair) {
+    if (k2 == 0 && (opt(kOptSmallTiles) < 0 ? small_wins(m, n, st) : opt(kOptSmallTiles) != 0)) {
+      using TS = SmallTraits<TIn, TOut, kNT, 0>;
+      return launch_small<TS>(small_plan<TS>(m, n, k, st), m, n, k, A, ldA, "A", B, ldB, "B", nullptr, 0, 1, C, ldC, alpha, beta, stream, st);
+    }
+  }
   constexpr int kBoxN = kPair ? T2::kBNHalf : T1::kBN;
   CUtensorMap ma, mb;
   int a3d = 0, b3d = 0;
@@ -746,14 +867,24 @@ int oft_ring(int m, int n, int k, int group_size, const void* A, int ldA, const 
 // is bound by shared-memory bandwidth, and every pair that rotates is one that does not multiply).  Interleaved
 // sustained runs, M 65536, K 8192, b 128, route 4 / route 3 time: N 28672 (2 pairs) 0.94, N 14336 (3 pairs) 0.93,
 // N 7168 (6 pairs) 0.98 to 1.02, N 3584 (7 pairs) 1.02; M 16384, K = N 4096, b 64 (6 pairs) 1.25.
+// 5: small_kernel (small_wins), which keeps the rotated slices in shared memory; needs no scratch, but only the routes
+// that may change with the scratch pool's presence (not the static entry point's) choose it.
 // Set by b200_oft_tn_f16_two_pass for its own call and by the option "oft_route".
 thread_local int g_oft_path = 0;
 
-int choose_route(int m, int group_size, int k, int b, const DeviceState* st) {
+// Groups small_kernel can take: its 128-column tiles must lie inside one group, and it takes no group that route 1 refuses.
+bool small_group_ok(int n, int group_size, int b) {
+  constexpr int kBN = CurrCompParams::bN;
+  return group_size == n || group_size % kBN == 0 || (group_size == 128 && kBN == 256 && b <= 64);
+}
+
+int choose_route(int m, int n, int group_size, int k, int b, const DeviceState* st) {
   int path = g_oft_path != 0 ? g_oft_path : opt(kOptOftRoute);
   const bool can_share = kOftPair && st->pool != nullptr;  // routes 2, 3 and 4 need scratch from the pool
-  if (path == 2 || path == 3 || path == 4) return can_share ? path : 1;
+  if (path == 2 || path == 3 || path == 4 || path == 5) return can_share ? path : 1;
   if (path == 1) return 1;
+  const int plan_m = g_plan_m > 0 ? g_plan_m : m, plan_n = g_plan_n > 0 ? g_plan_n : n;
+  if (can_share && opt(kOptSmallTiles) != 0 && small_group_ok(n, group_size, b) && small_wins(plan_m, plan_n, st)) return 5;
   const int min_tiles = b >= 128 ? 4 : 8;
   if (!can_share || group_size < min_tiles * static_cast<int>(CurrCompParams::bN)) return 1;
   if (g_more.n > 0) return 3;  // only oft3_kernel stores to further destinations
@@ -773,7 +904,7 @@ template <int kB>
 int launch_oft(int m, int n, int k, int group_size, const void* A, int ldA, const void* B, int ldB, const void* R, int ldR,
                void* C, int ldC, cudaStream_t stream, DeviceState* st) {
   constexpr int kBN = CurrCompParams::bN;
-  const int route = choose_route(m, group_size, k, kB, st);
+  const int route = choose_route(m, n, group_size, k, kB, st);
   if (route == 2) {
     const int rc = oft_two_pass<kB>(m, n, k, group_size, A, ldA, B, ldB, R, ldR, C, ldC, stream, st);
     if (rc != kNoScratch) return rc;
@@ -781,6 +912,10 @@ int launch_oft(int m, int n, int k, int group_size, const void* A, int ldA, cons
     // out of memory for X.R: the kernel that keeps X.R in tensor memory needs no scratch
   }
   if constexpr (kOftPair) {
+    if (route == 5 && small_group_ok(n, group_size, kB)) {
+      using TS = SmallTraits<__half, __half, false, kB>;
+      return launch_small<TS>(small_plan<TS>(n, m, k, st), n, m, k, B, ldB, "B", A, ldA, "A", R, ldR, group_size, C, ldC, 1.f, 0.f, stream, st);
+    }
     if ((route == 3 || route == 4) && (group_size == n || group_size % kBN == 0)) {
       const int rc = oft_ring<kB>(m, n, k, group_size, A, ldA, B, ldB, R, ldR, C, ldC, stream, st, route == 4);
       if (rc != kNoRing) return rc;
@@ -1106,8 +1241,10 @@ int b200_oft_plan(int m, int n, int k, int group_size, int reconn_sz, int* path,
     return fail(B200_EINVAL, "bad plan arguments (m=%d n=%d k=%d group_size=%d reconn_sz=%d)", m, n, k, group_size, reconn_sz);
   DeviceState* st;
   if (int rc = device_state(&st)) return rc;
-  const int route = choose_route(m, group_size, k, reconn_sz == 8 ? 16 : reconn_sz, st);
-  if (path) *path = route;
+  const int route = choose_route(m, n, group_size, k, reconn_sz == 8 ? 16 : reconn_sz, st);
+  // small_kernel forms X.R per tile of C on the chip and needs no scratch, like the kernel of route 1; a caller of the
+  // plan sees the same 1 for both unless it asked for 5 itself
+  if (path) *path = route == 5 && opt(kOptOftRoute) != 5 ? 1 : route;
   const int groups = n / group_size;
   if (kernel_launches) *kernel_launches = (route == 2 ? 2 * groups : ((route == 3 || route == 4) ? groups : 1)) + (reconn_sz == 8 ? 1 : 0);
   return B200_OK;
@@ -1145,6 +1282,7 @@ int b200_oft_tn_f16_host(int m, int n, int k, int group_size, int reconn_sz, con
   // i + 1, the product of chunk i and the download of chunk i - 1 overlap (the link is full duplex and the
   // download of Y is the longest leg: 3.76 GB against 1.55 GB up at M 65536, K 8192, N 28672).  Results do not
   // depend on the chunking: an element of Y only ever sees its own row of X and its own column of W.
+  const PlanAs whole(m, n);
   constexpr int kMaxChunks = 16;
   int chunk_rows = ((m + kMaxChunks - 1) / kMaxChunks + 255) & ~255;
   if (chunk_rows < 2048) chunk_rows = 2048;
@@ -1363,6 +1501,7 @@ int b200_oft_tn_f16_sharded(int m, int n, int k, int group_size, int reconn_sz, 
   int cur = 0;
   CUDA_TRY(cudaGetDevice(&cur));
   int rc = B200_OK;
+  const PlanAs whole(m, n);
   for (int r = 0; rc == B200_OK && r < world; ++r) {
     int n0 = 0, n1 = 0;
     rc = b200_shard_range(n, group_size, world, r, &n0, &n1);

@@ -98,13 +98,15 @@ __device__ __noinline__ void report_timeout(const WaitCtx& ctx, int site, uint32
 // caller then leaves its role loop and falls through to the common teardown.
 __device__ __forceinline__ bool mbar_wait_impl(uint32_t bar, uint32_t parity, const WaitCtx& ctx, int site) {
   if (mbar_try_wait(bar, parity)) return true;
-  const unsigned long long t0 = globaltimer_ns();
+  unsigned long long t0 = 0;
   int it = 0;
   while (true) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((++it & 63) == 0) {
       if (*ctx.abort_flag) return false;
-      if (globaltimer_ns() - t0 > ctx.limit_ns) {
+      const unsigned long long now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > ctx.limit_ns) {
         report_timeout(ctx, site, parity);
         return false;
       }
@@ -257,13 +259,15 @@ __device__ __forceinline__ bool mbar_try_wait_parked(uint32_t bar, uint32_t pari
 }
 __device__ __forceinline__ bool mbar_wait_parked_impl(uint32_t bar, uint32_t parity, const WaitCtx& ctx, int site) {
   if (mbar_try_wait(bar, parity)) return true;
-  const unsigned long long t0 = globaltimer_ns();
+  unsigned long long t0 = 0;
   int it = 0;
   while (true) {
     if (mbar_try_wait_parked(bar, parity, 20000u)) return true;
     if ((++it & 3) == 0) {
       if (*ctx.abort_flag) return false;
-      if (globaltimer_ns() - t0 > ctx.limit_ns) {
+      const unsigned long long now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > ctx.limit_ns) {
         report_timeout(ctx, site, parity);
         return false;
       }
@@ -284,9 +288,12 @@ __device__ __forceinline__ bool mbar_wait_parked(uint32_t bar, uint32_t parity, 
 }
 
 // Whole-warp form for roles whose next instruction is warp-collective (tcgen05.ld / st / wait): every lane gets
-// the same answer, so the warp stays converged when a wait gives up.  One lane waits (parked); the others then
-// look at the completed phase once, which gives each of them the barrier's acquire.
+// the same answer, so the warp stays converged when a wait gives up.  All lanes look first (in-kernel clock, wait
+// already complete: 230 cycles through the one-lane path below, 60 through the look); if that does not find the phase
+// complete, one lane waits (parked) and the others then look at the completed phase once, which gives each of them
+// the barrier's acquire.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, const WaitCtx& ctx, int site) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
   bool ok = true;
   if ((threadIdx.x & 31) == 0) ok = mbar_wait_parked(bar, parity, ctx, site);
   ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
@@ -296,6 +303,41 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, co
   return ok;
 }
 
+// Whole-warp wait for the roles the tensor pipe depends on: every lane polls, the answer is uniform.
+__device__ __forceinline__ bool mbar_wait_warp_spin(uint32_t bar, uint32_t parity, const WaitCtx& ctx, int site) {
+  unsigned long long t0 = 0;
+  int it = 0;
+  while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
+    if ((++it & 63) != 0) continue;
+    bool give_up = false;
+    if ((threadIdx.x & 31) == 0) {
+      const unsigned long long now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (*ctx.abort_flag) give_up = true;
+      else if (now - t0 > ctx.limit_ns) {
+        report_timeout(ctx, site, parity);
+        give_up = true;
+      }
+    }
+    if (__shfl_sync(0xffffffffu, give_up ? 1 : 0, 0) != 0) return false;
+  }
+  return true;
+}
+
+// One lane of the (converged) warp, always the same one.  Roles that issue tcgen05 or TMA instructions run their loops
+// with the whole warp and elect only around those instructions: descriptors and addresses then stay in uniform
+// registers.  Inside `if (lane == 0)` the compiler moves every operand over from ordinary registers instead (in-kernel
+// clock: 55 cycles per tcgen05.mma, whatever its size).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t pred;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(pred));
+  return pred != 0;
+}
+__device__ __forceinline__ int warp_id_uniform() { return __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0); }
+
 // Register re-balancing between warpgroups (all four warps of a warpgroup execute the same one).
 template <int kRegs> __device__ __forceinline__ void setmaxnreg_inc() {
   asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegs));
@@ -303,6 +345,11 @@ template <int kRegs> __device__ __forceinline__ void setmaxnreg_inc() {
 template <int kRegs> __device__ __forceinline__ void setmaxnreg_dec() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegs));
 }
+
+// Programmatic dependent launch: lets the next kernel of the stream start its prologue now / waits until the kernels
+// this one depends on have finished and their writes are visible.  Both are no-ops in a launch without the attribute.
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // ---- TMA ----------------------------------------------------------------------------------------
 // Tile store, shared memory (laid out as the tensor map's swizzle says) -> global; rows and columns past the

@@ -1,0 +1,129 @@
+"""small_kernel (problems with no more 128 x 128 tiles than SMs) at the edges of its tiles, its pieces along K and its
+rotation buffers, against the routes it replaces (bit for bit where K is not cut) and against fp64."""
+import numpy as np
+import pytest
+
+from _util import make_oft_case, truth_ok
+from cute_mma_b200 import ops
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _oft(lib, cuda, A, R, B, m, n, k, b, gs, ldc, shift, **opts):
+    """C[m, n] with rows ldc apart and its base `shift` elements past an aligned address; canaries around it."""
+    import contextlib
+    import torch
+
+    dA, dB, dR = (torch.from_numpy(x).to(cuda) for x in (A, B, R))
+    buf = torch.full(((m + 1) * ldc + shift,), -7.0, dtype=torch.float16, device=cuda)
+    with contextlib.ExitStack() as es:
+        for name, v in opts.items():
+            es.enter_context(ops.option(name, v, lib))
+        ops.oft_tn(m, n, k, dA, k, dB, k, dR, k, buf.data_ptr() + 2 * shift, ldc, group_size=gs, reconn_sz=b, lib=lib)
+        path = ops.oft_plan(m, n, k, group_size=gs, reconn_sz=b, lib=lib)["path"]
+    assert ops.device_status(lib)[0] == 0
+    out = buf.cpu().numpy()
+    rows = out[shift:].reshape(m + 1, ldc)
+    assert np.all(out[:shift] == -7.0) and np.all(rows[m] == -7.0) and np.all(rows[:m, n:] == -7.0)
+    return rows[:m, :n].copy(), path
+
+
+# rows at the edges of the 16-column granule, of a warp's 32 rows, of the three-buffer limit (64) and of a tile (128)
+@pytest.mark.parametrize("m,n,k,b,gs,pad,shift", [
+    (1, 256, 64, 64, None, 0, 0), (16, 300, 1024, 32, None, 4, 0), (17, 129, 1040, 16, None, 3, 1), (33, 512, 2048, 128, 256, 0, 0),
+    (64, 384, 1152, 64, 128, 8, 4), (65, 640, 1280, 128, None, 1, 0), (128, 127, 2056, 8, None, 0, 1), (129, 1000, 896, 32, None, 0, 0),
+    (257, 512, 8192, 128, 512, 0, 0), (300, 1280, 1344, 8, 256, 2, 0)])
+def test_small_oft_matches_the_other_route_and_truth(lib, cuda, pair_build, m, n, k, b, gs, pad, shift):
+    if not pair_build:
+        pytest.skip("the single-CTA build has one route")
+    A, R, B = make_oft_case(m, n, k, b, gs, seed=91, xdist="normal", wsigma=0.05)
+    args = (lib, cuda, A, R, B, m, n, k, b, gs, n + pad, shift)
+    got, _ = _oft(*args)
+    forced, path = _oft(*args, oft_route=5)
+    assert path == "fused_small" and np.array_equal(forced.view(np.uint16), got.view(np.uint16))  # the library's own choice
+    groups, g_sz = (1, n) if gs is None else (n // gs, gs)
+    truth = oracle.oft_f64(A, R, B, m, g_sz, groups, k, b, round_xr=True)
+    assert truth_ok(got, truth)[0] == 0
+    tmem, path = _oft(*args, oft_route=1)
+    assert path == "fused_tmem"
+    whole, _ = _oft(*args, oft_route=5, gemm_split=0)  # K in one piece: the same sums in the same order
+    assert np.array_equal(whole.view(np.uint16), tmem.view(np.uint16))
+    for split in (2, 3, 8):  # pieces of unequal length; one rounding of C, so at most a step of fp16 apart
+        cut, _ = _oft(*args, small_split=split)
+        d = np.abs(cut.astype(np.float64) - whole.astype(np.float64))
+        assert np.all(d <= 2.0 ** -10 * (np.abs(whole.astype(np.float64)) + 1.0)), (split, float(d.max()))
+
+
+@pytest.mark.parametrize("layout", ["TN", "NT"])
+@pytest.mark.parametrize("in_type,out_type", [(0, 0), (0, 1), (2, 1)])
+@pytest.mark.parametrize("m,n,k,alpha,beta,pad", [(1, 8, 8, 1.0, 0.0, 0), (129, 72, 1032, 1.0, 0.0, 1), (264, 136, 2048, 0.5, -0.25, 4), (120, 1000, 523, 1.0, 0.0, 3)])
+def test_small_gemm_matches_the_pair_kernel(lib, cuda, pair_build, layout, in_type, out_type, m, n, k, alpha, beta, pad):
+    if not pair_build:
+        pytest.skip("the small-problem kernel belongs to the CTA-pair build")
+    import torch
+
+    g = torch.Generator(device=cuda).manual_seed(92)
+    up8 = lambda x: (x + 7) // 8 * 8
+    tin, tout = (torch.float16 if in_type == 0 else torch.float32), (torch.float16 if out_type == 0 else torch.float32)
+    sa, sb = ((m, up8(k)), (n, up8(k))) if layout == "TN" else ((k, up8(m)), (k, up8(n)))
+    A, B = (torch.randn(s, generator=g, device=cuda).to(tin) for s in (sa, sb))
+    c0 = torch.randn((n + 1, m + pad), generator=g, device=cuda).to(tout)
+
+    def run(**opts):
+        C = c0.clone()
+        import contextlib
+        with contextlib.ExitStack() as es:
+            for name, v in opts.items():
+                es.enter_context(ops.option(name, v, lib))
+            ops.gemm_ex(*layout, m, n, k, alpha, A, sa[1], B, sb[1], beta, C, m + pad, in_type=in_type, out_type=out_type, lib=lib)
+        assert ops.device_status(lib)[0] == 0
+        assert torch.equal(C[n], c0[n]) and torch.equal(C[:, m:], c0[:, m:])
+        return C[:n, :m]
+
+    pair = run(small_tiles=0, gemm_split=0)
+    assert torch.equal(run(gemm_split=0), pair)
+    # cut along K: fp32 sums in another order, |error| <= K 2^-24 sum |a b| and one rounding of the result
+    bound = 4 * k ** 0.5 * 2.0 ** -23 + (2.0 ** -10 if out_type == 0 else 0)
+    scale = pair.double().abs() + abs(alpha) * k ** 0.5
+    for opts in ({}, {"small_split": 2}, {"small_split": 5}):
+        assert bool(((run(**opts).double() - pair.double()).abs() <= bound * scale).all()), opts
+
+
+def test_small_products_chained_on_two_streams(lib, cuda, pair_build):
+    """Launches that may start their prologue under the one before them: a chain in which every product reads what the
+    last one wrote, on two streams at once and under graph capture, gives the bits of the same chain with a
+    synchronisation after every launch."""
+    if not pair_build:
+        pytest.skip("the small-problem kernel belongs to the CTA-pair build")
+    import torch
+
+    n = k = 1024
+    g = torch.Generator(device=cuda).manual_seed(93)
+    W = (torch.randn((n, k), generator=g, device=cuda) / 32).half()
+    x0 = torch.randn((24, k), generator=g, device=cuda).half()
+
+    def chain(bufs, stream, wait=False):
+        for i in range(6):  # row-major [24][n]: the column-major n x 24 result of W . X^T
+            ops.gemm_tn(n, 24, k, W, k, bufs[i], k, bufs[i + 1], n, stream, lib=lib)
+            if wait:
+                torch.cuda.synchronize()
+
+    new = lambda: [x0.clone()] + [torch.zeros_like(x0) for _ in range(6)]
+    want = new()
+    chain(want, torch.cuda.current_stream(), wait=True)
+    s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+    b1, b2, b3 = new(), new(), new()
+    torch.cuda.synchronize()
+    for _ in range(3):
+        chain(b1, s1)
+        chain(b2, s2)
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        chain(b3, torch.cuda.current_stream())
+    graph.replay()
+    torch.cuda.synchronize()
+    assert ops.device_status(lib)[0] == 0
+    for b in (b1, b2, b3):
+        assert torch.equal(b[6], want[6])
