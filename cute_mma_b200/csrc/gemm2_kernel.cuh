@@ -67,7 +67,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   const long long kernel_c0 = clock64();
 #endif
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_id_uniform(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();  // 0 = leader (issues the MMAs), 1 = peer
   const unsigned pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   const unsigned tiles_m = (args.m + 2 * T::kBM - 1) / (2 * T::kBM), tiles_n = (args.n + T::kBN - 1) / T::kBN;
@@ -163,7 +163,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       // The issuing thread is on the critical path: measured with in-kernel cycle counters, every instruction
       // it executes between two MMAs shows up as idle time of the tensor pipe (a look at the next stage's
       // barrier whose address had to be computed: 512 -> 552 cycles per stage).  The ring is therefore walked
@@ -195,28 +195,37 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
           if (base + s >= total) break;
           if (ks == 0) {  // first K step of a tile: its accumulator must have been drained by the epilogue
             const int a = tcount % T::kAccBufs;
-            if (!(ok = mbar_wait(accempty_bar(a), ((tcount / T::kAccBufs) & 1) ^ 1, ctx, 2))) break;
+            if (!(ok = mbar_wait_warp_spin(accempty_bar(a), ((tcount / T::kAccBufs) & 1) ^ 1, ctx, 2))) break;
             d_tmem = tmem_base + a * T::kBN;
             if constexpr (kSplit) {
               const unsigned item = pair + tcount * num_pairs;
               steps_this = item_ks1(item) - item_ks0(item);
             }
           }
-          if (!have_full && !(ok = mbar_wait(full0 + 8 * s, phase, ctx, 3))) break;
+          if (!have_full && !(ok = mbar_wait_warp_spin(full0 + 8 * s, phase, ctx, 3))) break;
           tc_fence_after();
+          auto issue = [&](int kk0, int kk1) {
 #pragma unroll
-          for (int kk = 0; kk < T::kBK / T::kUmmaK; ++kk) {
-            if (kk == (T::kBK / T::kUmmaK) / 2)  // is the next stage there already?  (never waits; past the end it looks at a barrier nobody completes)
-              have_full = mbar_test_wait(full0 + 8 * ((s + 1) % T::kStages), s + 1 == T::kStages ? (phase ^ 1) : phase);
-            const uint32_t acc = (ks > 0 || kk > 0) ? 1u : 0u;
-            const uint64_t a_desc = a_desc0 + static_cast<uint64_t>((s * T::kStageBytes + kk * a_adv) >> 4);
-            const uint64_t b_desc = b_desc0 + static_cast<uint64_t>((s * T::kStageBytes + kk * b_adv) >> 4);
-            if constexpr (T::kFmt == kFmtF16) umma_f16_ss_pair(d_tmem, a_desc, b_desc, idesc, acc);
-            else umma_tf32_ss_pair(d_tmem, a_desc, b_desc, idesc, acc);
+            for (int kk = kk0; kk < kk1; ++kk) {
+              const uint32_t acc = (ks > 0 || kk > 0) ? 1u : 0u;
+              const uint64_t a_desc = a_desc0 + static_cast<uint64_t>((s * T::kStageBytes + kk * a_adv) >> 4);
+              const uint64_t b_desc = b_desc0 + static_cast<uint64_t>((s * T::kStageBytes + kk * b_adv) >> 4);
+              if constexpr (T::kFmt == kFmtF16) umma_f16_ss_pair(d_tmem, a_desc, b_desc, idesc, acc);
+              else umma_tf32_ss_pair(d_tmem, a_desc, b_desc, idesc, acc);
+            }
+          };
+          constexpr int kSlices = T::kBK / T::kUmmaK;
+          if (elect_one()) issue(0, kSlices / 2);
+          // is the next stage there already?  (never waits; past the end it looks at a barrier nobody completes)
+          have_full = mbar_test_warp(full0 + 8 * ((s + 1) % T::kStages), s + 1 == T::kStages ? (phase ^ 1) : phase);
+          const bool tile_ends = ks + 1 == (kSplit ? steps_this : k_steps);
+          if (elect_one()) {
+            issue(kSlices / 2, kSlices);
+            umma_commit_pair(empty0 + 8 * s, 3);  // frees the stage in both CTAs
+            if (tile_ends) umma_commit_pair(accfull_bar(tcount % T::kAccBufs), 3);
           }
-          umma_commit_pair(empty0 + 8 * s, 3);  // frees the stage in both CTAs
-          if (++ks == (kSplit ? steps_this : k_steps)) {
-            umma_commit_pair(accfull_bar(tcount % T::kAccBufs), 3);
+          ++ks;
+          if (tile_ends) {
             ks = 0;
             ++tcount;
           }

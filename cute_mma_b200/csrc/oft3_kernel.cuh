@@ -143,7 +143,7 @@ oft3_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
   if (threadIdx.x == 0) skew_stamp(ctx, kSkewTiles - 2);  // when this CTA started
 #endif
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_id_uniform(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const unsigned pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   const unsigned tiles_m = (args.m + 2 * T::kBM - 1) / (2 * T::kBM), tiles_n = (args.n + T::kBN - 1) / T::kBN;
@@ -270,21 +270,22 @@ oft3_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
   } else if (warp == 2) {
     // -------------------------------------------------------------- issuer of the rotation MMAs (leader CTA only)
     setmaxnreg_dec<112>();
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       constexpr uint32_t idesc1 = umma_idesc(kFmtF16, 0, 0, 2 * T::kBM, T::kB);
       const uint64_t x_desc0 = umma_desc_sw128(ring1, 16, 1024), r_desc0 = umma_desc_sw128(ring1 + T::kXBytes, 16, 1024);
       uint32_t it = 0;
       bool ok = true;
       for (unsigned i = 0; ok && i < my_units; ++i) {
         const int xb = i % T::kXrBufs;
-        if (!(ok = mbar_wait_parked(x_empty + 8 * xb, ((i / T::kXrBufs) & 1) ^ 1, ctx, 20))) break;
+        if (!(ok = mbar_wait_warp_spin(x_empty + 8 * xb, ((i / T::kXrBufs) & 1) ^ 1, ctx, 20))) break;
         const uint32_t d1 = tmem_base + T::kColXr + xb * T::kUnitK;
         for (int su = 0; su < T::kStagesPerUnit; ++su, ++it) {
           const int s = it % T::kS1;
-          if (!(ok = mbar_wait_parked(full1 + 8 * s, (it / T::kS1) & 1, ctx, 21))) break;
+          if (!(ok = mbar_wait_warp_spin(full1 + 8 * s, (it / T::kS1) & 1, ctx, 21))) break;
           tc_fence_after();
           const uint64_t x_desc = x_desc0 + static_cast<uint64_t>(s * (T::kS1Bytes >> 4));
           const uint64_t r_desc = r_desc0 + static_cast<uint64_t>(s * (T::kS1Bytes >> 4));
+          if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < T::kBK / 16; ++kk) {
             // b < 64: the stage holds 64/b diagonal blocks; slice kk belongs to block (kk*16)/b and lands in
@@ -294,18 +295,20 @@ oft3_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
             const uint32_t accum = small ? ((((kk * 16) % T::kB) != 0) ? 1u : 0u) : ((su > 0 || kk > 0) ? 1u : 0u);
             umma_f16_ss_pair(d1 + blk * T::kB, x_desc + kk * 2, r_desc + kk * 2, idesc1, accum);
           }
-          umma_commit_pair(empty1 + 8 * s, 3);
+            umma_commit_pair(empty1 + 8 * s, 3);
+            if (su == T::kStagesPerUnit - 1) umma_commit_pair(x_acc + 8 * xb, 3);  // the rotation epilogues of both CTAs start on their halves
+          }
+          __syncwarp();
         }
         if (!ok) break;
         early_stamp(ctx, i, 1);
-        umma_commit_pair(x_acc + 8 * xb, 3);  // the rotation epilogues of both CTAs start on their halves
       }
     }
     __syncwarp();
   } else if (warp == 3) {
     // -------------------------------------------------------------- issuer of the product MMAs (leader CTA only)
     setmaxnreg_dec<112>();
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       // Unrolled over the ring's stages with the tiles flattened into one stream of K steps (every barrier
       // address, parity and descriptor offset is a constant plus a base register), like the plain pair GEMM.
       constexpr uint32_t idesc2 = umma_idesc(kFmtF16, 0, 0, 2 * T::kBM, T::kBN);
@@ -320,27 +323,35 @@ oft3_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
         for (int s = 0; s < T::kS2; ++s) {
           if (base + s >= total) break;
           if (ks == 0) {  // first K step of a tile: the epilogue must have drained the accumulator
-            if (!(ok = mbar_wait(acc_empty, (tcount & 1) ^ 1, ctx, 22))) break;
+            if (!(ok = mbar_wait_warp_spin(acc_empty, (tcount & 1) ^ 1, ctx, 22))) break;
           }
-          if (!have_full && !(ok = mbar_wait(full2 + 8 * s, phase, ctx, 24))) break;
+          if (!have_full && !(ok = mbar_wait_warp_spin(full2 + 8 * s, phase, ctx, 24))) break;
           tc_fence_after();
+          auto issue = [&](int kk0, int kk1) {
 #pragma unroll
-          for (int kk = 0; kk < T::kBK / 16; ++kk) {
-            if (kk == 2)  // is the next stage there already?  (never waits)
-              have_full = mbar_test_wait(full2 + 8 * ((s + 1) % T::kS2), s + 1 == T::kS2 ? (phase ^ 1) : phase);
-            const uint32_t acc = (ks > 0 || kk > 0) ? 1u : 0u;
-            const uint64_t a_desc = a_desc0 + static_cast<uint64_t>((s * T::kS2Bytes + kk * 32) >> 4);
-            const uint64_t b_desc = b_desc0 + static_cast<uint64_t>((s * T::kS2Bytes + kk * 32) >> 4);
-            umma_f16_ss_pair(d_tmem, a_desc, b_desc, idesc2, acc);
+            for (int kk = kk0; kk < kk1; ++kk) {
+              const uint32_t acc = (ks > 0 || kk > 0) ? 1u : 0u;
+              const uint64_t a_desc = a_desc0 + static_cast<uint64_t>((s * T::kS2Bytes + kk * 32) >> 4);
+              const uint64_t b_desc = b_desc0 + static_cast<uint64_t>((s * T::kS2Bytes + kk * 32) >> 4);
+              umma_f16_ss_pair(d_tmem, a_desc, b_desc, idesc2, acc);
+            }
+          };
+          if (elect_one()) issue(0, 2);
+          // is the next stage there already?  (never waits)
+          have_full = mbar_test_warp(full2 + 8 * ((s + 1) % T::kS2), s + 1 == T::kS2 ? (phase ^ 1) : phase);
+          const bool tile_ends = ks + 1 == k_steps;
+          if (elect_one()) {
+            issue(2, 4);
+            umma_commit_pair(empty2 + 8 * s, 3);  // frees the stage in both CTAs
+            if (tile_ends) umma_commit_pair(acc_full, 3);
           }
-          umma_commit_pair(empty2 + 8 * s, 3);  // frees the stage in both CTAs
-          if (++ks == k_steps) {
-            umma_commit_pair(acc_full, 3);
+          ++ks;
+          if (tile_ends) {
             ks = 0;
             ++tcount;
           }
         }
-        phase ^= 1;
+      phase ^= 1;
       }
     }
     __syncwarp();

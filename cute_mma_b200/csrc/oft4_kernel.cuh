@@ -158,19 +158,20 @@ __device__ __forceinline__ bool oft4_rotate(int warp, int lane, uint32_t rank, B
     __syncwarp();
   } else if (warp == 1) {
     // -------------------------------------------------------------- issuer of the rotation MMAs (leader CTA only)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       constexpr uint32_t idesc1 = umma_idesc(kFmtF16, 0, 0, 2 * T::kBM, T::kB);
       const uint64_t x_desc0 = umma_desc_sw128(sm.ring1, 16, 1024), r_desc0 = umma_desc_sw128(sm.ring1 + T::kXBytes, 16, 1024);
       for (; ok && share.next(xb, ku); ++st.i) {
         const int buf = st.i % T::kXrBufs;
-        if (!(ok = mbar_wait(sm.x_empty + 8 * buf, ((st.i / T::kXrBufs) & 1) ^ 1, ctx, 20))) break;
+        if (!(ok = mbar_wait_warp_spin(sm.x_empty + 8 * buf, ((st.i / T::kXrBufs) & 1) ^ 1, ctx, 20))) break;
         const uint32_t d1 = sm.tmem_base + buf * T::kUnitK;
         for (int su = 0; su < T::kStagesPerUnit; ++su, ++st.it) {
           const int s = st.it % T::kS1;
-          if (!(ok = mbar_wait(sm.full1 + 8 * s, (st.it / T::kS1) & 1, ctx, 21))) break;
+          if (!(ok = mbar_wait_warp_spin(sm.full1 + 8 * s, (st.it / T::kS1) & 1, ctx, 21))) break;
           tc_fence_after();
           const uint64_t x_desc = x_desc0 + static_cast<uint64_t>(s * (T::kS1Bytes >> 4));
           const uint64_t r_desc = r_desc0 + static_cast<uint64_t>(s * (T::kS1Bytes >> 4));
+          if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < T::kBK / 16; ++kk) {
             // b < 64: the stage holds 64/b diagonal blocks; slice kk belongs to block (kk*16)/b and lands in
@@ -180,10 +181,12 @@ __device__ __forceinline__ bool oft4_rotate(int warp, int lane, uint32_t rank, B
             const uint32_t accum = small ? ((((kk * 16) % T::kB) != 0) ? 1u : 0u) : ((su > 0 || kk > 0) ? 1u : 0u);
             umma_f16_ss_pair(d1 + blk * T::kB, x_desc + kk * 2, r_desc + kk * 2, idesc1, accum);
           }
-          umma_commit_pair(sm.empty1 + 8 * s, 3);
+            umma_commit_pair(sm.empty1 + 8 * s, 3);
+            if (su == T::kStagesPerUnit - 1) umma_commit_pair(sm.x_acc + 8 * buf, 3);  // the rotation epilogues of both CTAs start on their halves
+          }
+          __syncwarp();
         }
         if (!ok) break;
-        umma_commit_pair(sm.x_acc + 8 * buf, 3);  // the rotation epilogues of both CTAs start on their halves
       }
     }
     __syncwarp();
@@ -286,7 +289,7 @@ oft4_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
   volatile unsigned* seen_tile = reinterpret_cast<volatile unsigned*>(tmem_slot + 3);  // tile whose X.R rows the epilogue saw ready
   const WaitCtx ctx{abort_flag, args.status, kWaitLimitNs};
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_id_uniform(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const unsigned pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   const unsigned rot_pairs = static_cast<unsigned>(args.rot_pairs), prod_pairs = num_pairs - rot_pairs;
@@ -380,7 +383,7 @@ oft4_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
       __syncwarp();
     } else if (warp == 1) {
       // ------------------------------------------------------------ product pair: MMA issuer (leader CTA only)
-      if (lane == 0 && rank == 0) {
+      if (rank == 0) {
         // The ring is walked in a loop unrolled over its stages with the tiles flattened into one stream of K
         // steps: every barrier address, parity and descriptor offset is a constant plus a base register.
         constexpr uint32_t idesc = umma_idesc(kFmtF16, 0, 0, 2 * T::kBM, T::kBN);
@@ -397,28 +400,36 @@ oft4_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
             if (base + s >= total) break;
             if (ks == 0) {  // first K step of a tile: its accumulator must have been drained by the epilogue
               const int a = tcount % T::kAccBufs;
-              if (!(ok = mbar_wait(accempty + 8 * a, ((tcount / T::kAccBufs) & 1) ^ 1, ctx, 22))) break;
+              if (!(ok = mbar_wait_warp_spin(accempty + 8 * a, ((tcount / T::kAccBufs) & 1) ^ 1, ctx, 22))) break;
               d_tmem = tmem_base + a * T::kBN;
             }
-            if (!have_full && !(ok = mbar_wait(full + 8 * s, phase, ctx, 24))) break;
+            if (!have_full && !(ok = mbar_wait_warp_spin(full + 8 * s, phase, ctx, 24))) break;
             tc_fence_after();
+            auto issue = [&](int kk0, int kk1) {
 #pragma unroll
-            for (int kk = 0; kk < T::kBK / 16; ++kk) {
-              if (kk == 2)  // is the next stage there already?  (never waits)
-                have_full = mbar_test_wait(full + 8 * ((s + 1) % T::kStages), s + 1 == T::kStages ? (phase ^ 1) : phase);
-              const uint32_t acc = (ks > 0 || kk > 0) ? 1u : 0u;
-              const uint64_t a_desc = a_desc0 + static_cast<uint64_t>((s * T::kStageBytes + kk * 32) >> 4);
-              const uint64_t b_desc = b_desc0 + static_cast<uint64_t>((s * T::kStageBytes + kk * 32) >> 4);
-              umma_f16_ss_pair(d_tmem, a_desc, b_desc, idesc, acc);
+              for (int kk = kk0; kk < kk1; ++kk) {
+                const uint32_t acc = (ks > 0 || kk > 0) ? 1u : 0u;
+                const uint64_t a_desc = a_desc0 + static_cast<uint64_t>((s * T::kStageBytes + kk * 32) >> 4);
+                const uint64_t b_desc = b_desc0 + static_cast<uint64_t>((s * T::kStageBytes + kk * 32) >> 4);
+                umma_f16_ss_pair(d_tmem, a_desc, b_desc, idesc, acc);
+              }
+            };
+            if (elect_one()) issue(0, 2);
+            // is the next stage there already?  (never waits)
+            have_full = mbar_test_warp(full + 8 * ((s + 1) % T::kStages), s + 1 == T::kStages ? (phase ^ 1) : phase);
+            const bool tile_ends = ks + 1 == k_steps;
+            if (elect_one()) {
+              issue(2, 4);
+              umma_commit_pair(empty + 8 * s, 3);  // frees the stage in both CTAs
+              if (tile_ends) umma_commit_pair(accfull + 8 * (tcount % T::kAccBufs), 3);
             }
-            umma_commit_pair(empty + 8 * s, 3);  // frees the stage in both CTAs
-            if (++ks == k_steps) {
-              umma_commit_pair(accfull + 8 * (tcount % T::kAccBufs), 3);
+            ++ks;
+            if (tile_ends) {
               ks = 0;
               ++tcount;
             }
           }
-          phase ^= 1;
+        phase ^= 1;
         }
       }
       __syncwarp();

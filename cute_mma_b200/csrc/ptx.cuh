@@ -336,6 +336,8 @@ __device__ __forceinline__ bool elect_one() {
       : "=r"(pred));
   return pred != 0;
 }
+// mbar_test_wait by a whole warp, one answer.
+__device__ __forceinline__ bool mbar_test_warp(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_test_wait(bar, parity)); }
 __device__ __forceinline__ int warp_id_uniform() { return __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0); }
 
 // Register re-balancing between warpgroups (all four warps of a warpgroup execute the same one).

@@ -59,7 +59,7 @@ xr_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CU
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const WaitCtx ctx{abort_flag, args.status, kWaitLimitNs};
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_id_uniform(), lane = threadIdx.x & 31;
   const unsigned tiles_m = (args.m + T::kBM - 1) / T::kBM;
   const unsigned units = (args.k + T::kUnitK - 1) / T::kUnitK;
   const unsigned num_units = tiles_m * units;
@@ -105,21 +105,22 @@ xr_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CU
     __syncwarp();
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    {
       constexpr uint32_t idesc = umma_idesc(kFmtF16, 0, 0, T::kBM, T::kB);
       const uint64_t a_desc0 = umma_desc_sw128(ring, 16, 1024), r_desc0 = umma_desc_sw128(ring + T::kABytes, 16, 1024);
       uint32_t it = 0;
       bool ok = true;
       for (unsigned g = 0; ok && g < my_units; ++g) {
         const int buf = g % T::kBufs;
-        if (!(ok = mbar_wait(x_empty + 8 * buf, ((g / T::kBufs) & 1) ^ 1, ctx, 25))) break;
+        if (!(ok = mbar_wait_warp_spin(x_empty + 8 * buf, ((g / T::kBufs) & 1) ^ 1, ctx, 25))) break;
         const uint32_t d = tmem_base + buf * T::kUnitK;
         for (int su = 0; su < T::kStagesPerUnit; ++su, ++it) {
           const int s = it % T::kS;
-          if (!(ok = mbar_wait(full + 8 * s, (it / T::kS) & 1, ctx, 26))) break;
+          if (!(ok = mbar_wait_warp_spin(full + 8 * s, (it / T::kS) & 1, ctx, 26))) break;
           tc_fence_after();
           const uint64_t a_desc = a_desc0 + static_cast<uint64_t>(s * (T::kSBytes >> 4));
           const uint64_t r_desc = r_desc0 + static_cast<uint64_t>(s * (T::kSBytes >> 4));
+          if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < T::kBK / 16; ++kk) {
             // b < 64: the stage holds 64/b diagonal blocks; slice kk belongs to block (kk*16)/b and lands in
@@ -129,10 +130,11 @@ xr_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CU
             const uint32_t accum = small ? ((((kk * 16) % T::kB) != 0) ? 1u : 0u) : ((su > 0 || kk > 0) ? 1u : 0u);
             umma_f16_ss(d + blk * T::kB, a_desc + kk * 2, r_desc + kk * 2, idesc, accum);
           }
-          umma_commit(empty + 8 * s);
+            umma_commit(empty + 8 * s);
+            if (su == T::kStagesPerUnit - 1) umma_commit(x_full + 8 * buf);
+          }
+          __syncwarp();
         }
-        if (!ok) break;
-        umma_commit(x_full + 8 * buf);
       }
     }
     __syncwarp();
