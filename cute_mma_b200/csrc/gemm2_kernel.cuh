@@ -245,7 +245,6 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
     uint32_t tcount = 0;
     bool ok = true;
     TOut* C = reinterpret_cast<TOut*>(args.C);
-    const bool scaled = args.alpha != 1.f || args.beta != 0.f;
     for (unsigned item = pair; ok && item < num_items; item += num_pairs, ++tcount) {
       const unsigned tile = item_tile(item);
       unsigned tm, tn;
@@ -255,6 +254,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
       tc_fence_after();
       const int row = tm * 2 * T::kBM + rank * T::kBM + quad * 32 + lane;
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + a * T::kBN;
+      const bool fast = k_steps < kLongTile || item + num_pairs >= num_items;
       if constexpr (kSplit) {
         if (item >= args.split_first) {
           // A piece of a split tile: park the fp32 partial tile (groups of four columns per row, so a thread moves
@@ -324,21 +324,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
         tmem_ld_x32(t_row + c * 32, v);
         tmem_wait_ld();
         const int col0 = tn * T::kBN + c * 32;
-        if (row < args.m) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            if (col0 + j < args.n) {
-              float f = __uint_as_float(v[j]);
-              TOut* dst = C + row + static_cast<long long>(col0 + j) * args.ldC;
-              if (scaled) {  // C = alpha * A.B^T + beta * C (the epilogue the reference leaves as a stub, gemm_tc.hpp:241)
-                f *= args.alpha;
-                if (args.beta != 0.f) f += args.beta * static_cast<float>(*dst);
-              }
-              if constexpr (sizeof(TOut) == 2) *dst = __float2half_rn(f);
-              else *dst = f;
-            }
-          }
-        }
+        if (row < args.m)
+          store_columns<TOut>(v, C + row + static_cast<long long>(col0) * args.ldC, args.ldC, args.n - col0, args.alpha, args.beta, fast);
       }
       tc_fence_before();
       mbar_arrive_cluster(mapa_shared(accempty_bar(a), 0));  // the leader's barrier collects both CTAs

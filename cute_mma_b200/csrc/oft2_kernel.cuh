@@ -457,11 +457,16 @@ oft2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       tc_fence_before();
       mbar_arrive_cluster(mapa_shared(acc_empty, 0));
       if (threadIdx.x == 256) skew_stamp(ctx, tcount);
-      if (row < args.m) {
+      if (!vec_ok) {  // rows not 16-byte aligned: 128 bytes of one row per instruction (see warp_store_rows)
+        warp_transpose_words<T::kBN / 64>(p, lane);
+        const int row0 = tm * 2 * T::kBM + rank * T::kBM + quad * 32;
+        warp_store_rows<T::kBN / 64>(p, args.C + static_cast<long long>(row0) * args.ldC + tn * T::kBN, args.ldC, args.m - row0,
+                                     args.n - static_cast<int>(tn) * T::kBN, lane);
+      } else if (row < args.m) {
 #pragma unroll
         for (int c = 0; c < T::kBN / 32; ++c) {
           const int col0 = tn * T::kBN + c * 32;
-          if (vec_ok && col0 + 32 <= args.n) {
+          if (col0 + 32 <= args.n) {
             uint4* dst = reinterpret_cast<uint4*>(c_row + col0);
 #pragma unroll
             for (int q = 0; q < 4; ++q)

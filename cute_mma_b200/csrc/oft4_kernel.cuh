@@ -457,11 +457,8 @@ oft4_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
           tmem_ld_x32(t_row + c * 32, v);
           tmem_wait_ld();
           const int xrow0 = xb * 2 * T::kBM + c * 32;
-          if (ycol < args.n) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (xrow0 + j < args.m) out[static_cast<long long>(xrow0 + j) * args.ldC] = __float2half_rn(__uint_as_float(v[j]));
-          }
+          if (ycol < args.n) store_columns<__half>(v, out + static_cast<long long>(xrow0) * args.ldC, args.ldC, args.m - xrow0, 1.f, 0.f,
+                                                   k_steps < kLongTile || tile + prod_pairs >= num_tiles);
         }
         tc_fence_before();
         mbar_arrive_cluster(mapa_shared(accempty + 8 * a, 0));  // the leader's barrier collects both CTAs

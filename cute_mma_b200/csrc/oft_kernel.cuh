@@ -15,7 +15,7 @@
 // MMA1 runs ahead of MMA2 by as many units as there are XR buffers in tensor memory, so the conversion of
 // the next units overlaps the main contraction.  All hand-offs are mbarriers with bounded waits.
 #pragma once
-#include "ptx.cuh"
+#include "gemm_kernel.cuh"
 
 namespace b200 {
 

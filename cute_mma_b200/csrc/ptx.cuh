@@ -590,6 +590,64 @@ __host__ __device__ constexpr uint32_t umma_idesc(int fmt, int a_mn_major, int b
 constexpr int kFmtF16 = 0;
 constexpr int kFmtTF32 = 2;
 
+// ---- row-major stores of a warp's 32 rows ---------------------------------------------------------------
+// p[blk * 32 + j] of lane r holds row r's columns 64 blk + 2 j, + 1 (two fp16).  A lane that stores its own row touches
+// 32 different rows per instruction: fine in 16-byte pieces, 32 sectors per 2-byte element when rows are not 16-byte
+// aligned.  The transpose (a butterfly of lane exchanges, 32 x 32 words at a time) turns this into
+// p[blk * 32 + i] of lane L = word L of row i's block, so that one instruction writes 128 contiguous bytes of one row.
+template <int kBlocks>
+__device__ __forceinline__ void warp_transpose_words(uint32_t (&p)[kBlocks * 32], int lane) {
+#pragma unroll
+  for (int blk = 0; blk < kBlocks; ++blk) {
+#pragma unroll
+    for (int sft = 16; sft >= 1; sft >>= 1) {
+      const bool upper = (lane & sft) != 0;
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        if (j & sft) continue;
+        uint32_t& lo = p[blk * 32 + j];
+        uint32_t& hi = p[blk * 32 + j + sft];
+        const uint32_t got = __shfl_xor_sync(0xFFFFFFFFu, upper ? lo : hi, sft);
+        if (upper) lo = got; else hi = got;
+      }
+    }
+  }
+}
+// Stores transposed words to `rows` rows of `cols` columns at base (any 2-byte aligned address and leading dimension).
+// In a row that starts between two words, every lane takes the second half of its own word and the first of its
+// neighbour's.
+template <int kBlocks>
+__device__ __forceinline__ void warp_store_rows(const uint32_t (&p)[kBlocks * 32], __half* base, long long ld, int rows, int cols, int lane) {
+#pragma unroll
+  for (int i = 0; i < 32; ++i) {
+    if (i >= rows) break;
+    __half* row = base + i * ld;
+    if ((reinterpret_cast<uintptr_t>(row) & 2) == 0) {
+#pragma unroll
+      for (int blk = 0; blk < kBlocks; ++blk) {
+        const int c = blk * 64 + 2 * lane;
+        const uint32_t w = p[blk * 32 + i];
+        if (c + 1 < cols) *reinterpret_cast<uint32_t*>(row + c) = w;
+        else if (c < cols) row[c] = __ushort_as_half(static_cast<unsigned short>(w & 0xFFFFu));
+      }
+    } else {
+      if (lane == 0) row[0] = __ushort_as_half(static_cast<unsigned short>(p[i] & 0xFFFFu));
+#pragma unroll
+      for (int blk = 0; blk < kBlocks; ++blk) {
+        const int c = blk * 64 + 2 * lane + 1;
+        const uint32_t w = p[blk * 32 + i];
+        uint32_t next = __shfl_down_sync(0xFFFFFFFFu, w, 1);
+        if (blk + 1 < kBlocks) {
+          const uint32_t first = __shfl_sync(0xFFFFFFFFu, p[(blk + 1 < kBlocks ? blk + 1 : blk) * 32 + i], 0);
+          if (lane == 31) next = first;
+        }
+        if (c + 1 < cols && c + 1 < kBlocks * 64) *reinterpret_cast<uint32_t*>(row + c) = (w >> 16) | (next << 16);
+        else if (c < cols) row[c] = __ushort_as_half(static_cast<unsigned short>(w >> 16));
+      }
+    }
+  }
+}
+
 // ---- tile rasteriser -------------------------------------------------------------------------------
 // Linear tile id -> (m, n) tile coordinate.  Same visiting order as the reference's z_curve
 // (z_curve.hpp:4-49): the grid is factored level by level by the smallest prime factor of what is

@@ -22,7 +22,7 @@
 //   MMA2  acc[128 x n_tile] += W[128 x 64] . XR^T
 // MMA1 runs up to xbufs slices ahead of MMA2, so the conversion is off the tensor pipe's path.
 #pragma once
-#include "ptx.cuh"
+#include "gemm_kernel.cuh"
 
 namespace b200 {
 
@@ -307,9 +307,7 @@ small_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_constant__
           for (int j = 0; j < 32; ++j)
             if (c + j < cols) asm volatile("st.shared.b32 [%0], %1;" ::"r"(dst + j * 512), "r"(v[j]) : "memory");
         } else if (m0 + r < args.m) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (c + j < cols) store(__uint_as_float(v[j]), C + (m0 + r) + static_cast<long long>(n0 + c + j) * args.ldC);
+          store_columns<TOut>(v, C + (m0 + r) + static_cast<long long>(n0 + c) * args.ldC, args.ldC, cols - c, args.alpha, args.beta, true);
         }
       }
     }
