@@ -295,11 +295,26 @@ struct PlanAs {
 // Tiles of 128 x 128 of an m x n result.
 long long tiles_128(int m, int n) { return ((static_cast<long long>(m) + 127) / 128) * ((static_cast<long long>(n) + 127) / 128); }
 
-// Whether small_kernel takes an m x n result: as long as its 128 x 128 tiles do not outnumber the SMs.  Below the line
-// every one of 150 random shapes of the operator surface ran faster on it than on the pair kernels, by 1.1 to 6.7 times
-// (fixed cost per launch 5 us against 9 to 10 us, and 256 x 256 tiles leave most SMs idle: 8 x 4096 x 4096 OFT 35 -> 10
-// us, 640 x 1280 x 1024 TF32 29 -> 10 us); above it long K is the pair kernels' (2808 x 968 x 9590: 82 against 123 us).
-bool small_wins(int m, int n, const DeviceState* st) { return tiles_128(m, n) <= st->sm_count; }
+// Products whose K range must not be cut (the parts of a two-pass product, see oft_two_pass).
+thread_local bool g_whole_k = false;
+
+// Whether small_kernel takes a plain m x n product of `steps` K steps (128 bytes of a row each).
+// As long as its 128 x 128 tiles do not outnumber the SMs, always: every one of 150 random shapes of the operator
+// surface ran faster on it than on the pair kernels, by 1.1 to 6.7 times (fixed cost per launch 5 us against 9 to 12 us,
+// and 256 x 256 tiles leave most SMs idle: 640 x 1280 x 1024 TF32 29 -> 10 us).  Above, the two are compared by a model
+// fitted to 120 random shapes: a round of pair tiles costs 0.36 us per K step on 74 pairs, two small tiles per SM cost
+// 0.72 us per step between them (both operands of a 128-wide tile are read from shared memory at its full rate), plus
+// the fixed costs and 1.5 us of epilogue per round.  1848 x 1488 x 489 half: 8.9 against 12.8 us; 2904 x 960 x 11305: 110
+// against 70 us.
+bool small_wins(int m, int n, int steps, const DeviceState* st) {
+  const long long t128 = tiles_128(m, n), pairs = st->sm_count / 2;
+  if (t128 <= st->sm_count) return true;
+  const long long t256 = ((static_cast<long long>(m) + 255) / 256) * ((static_cast<long long>(n) + 255) / 256);
+  const double rounds = static_cast<double>(t128) / (2.0 * st->sm_count);
+  const double small = 5.0 + (rounds > 1.0 ? rounds : 1.0) * (0.72 * steps + 1.5);
+  const double pair = 11.5 + static_cast<double>((t256 + pairs - 1) / pairs) * (0.36 * steps + 1.5);
+  return small < pair;
+}
 
 struct SmallPlan {
   int tiles_m, tiles_n, n_tile, split, stages, xbufs, smem;
@@ -425,7 +440,7 @@ int launch_gemm_bn(int m, int n, int k, const void* A, int ldA, const void* B, i
   DeviceState* st;
   if (int rc = device_state(&st)) return rc;
   if constexpr (kPair) {
-    if (k2 == 0 && (opt(kOptSmallTiles) < 0 ? small_wins(m, n, st) : opt(kOptSmallTiles) != 0)) {
+    if (k2 == 0 && !g_whole_k && (opt(kOptSmallTiles) < 0 ? small_wins(m, n, (k + T1::kBK - 1) / T1::kBK, st) : opt(kOptSmallTiles) != 0)) {
       using TS = SmallTraits<TIn, TOut, kNT, 0>;
       return launch_small<TS>(small_plan<TS>(m, n, k, st), m, n, k, A, ldA, "A", B, ldB, "B", nullptr, 0, 1, C, ldC, alpha, beta, stream, st);
     }
@@ -487,7 +502,7 @@ int launch_gemm_bn(int m, int n, int k, const void* A, int ldA, const void* B, i
     long long parts = (rest > 0 && rest * 2 <= all_pairs && full_waves == 0 && !big && st->pool) ? all_pairs / rest : 1;
     if (parts > 4) parts = 4;
     if (parts > k_steps_all / 8) parts = k_steps_all / 8;
-    if (opt(kOptGemmSplit) == 0 || alpha != 1.f || beta != 0.f) parts = 1;  // the split instance sums pieces, it does not scale
+    if (opt(kOptGemmSplit) == 0 || g_whole_k || alpha != 1.f || beta != 0.f) parts = 1;  // the split instance sums pieces, it does not scale
     if (parts >= 2) {
       void* scratch = nullptr;
       const size_t tile_floats = static_cast<size_t>(T2::kBM) * T2::kBN;
@@ -645,25 +660,45 @@ int launch_xr(int m, int k, const void* A, int ldA, const void* Rg, int ldR, voi
 
 constexpr int kNoScratch = -1000;  // internal: no device memory for X.R
 
+//
+// The library takes this route by itself (`own`) where the fused kernels are held up: rows of C that are not 16-byte
+// aligned, which the GEMM's epilogue stores along N whatever their alignment, and short K, where a ring kernel's
+// hand-off of X.R (about 2 us per row block) and its single accumulator show.  Then X.R is formed for at most
+// kOwnScratch bytes of rows at a time and the GEMM's K range is never cut, so that the bits are those of the routes
+// it stands in for.
+constexpr size_t kOwnScratch = size_t(256) << 20;
+long long two_pass_rows(int m, int k, bool own) {  // rows of X.R formed at a time
+  const size_t row_bytes = static_cast<size_t>((k + 7) & ~7) * 2;
+  if (!own || static_cast<size_t>(m) * row_bytes <= kOwnScratch) return m;
+  const long long most = static_cast<long long>(kOwnScratch / row_bytes) / 256 * 256, chunks = (m + most - 1) / most;
+  return ((m + chunks - 1) / chunks + 255) / 256 * 256;  // equal chunks
+}
 template <int kB>
 int oft_two_pass(int m, int n, int k, int group_size, const void* A, int ldA, const void* B, int ldB, const void* R, int ldR,
-                 void* C, int ldC, cudaStream_t stream, DeviceState* st) {
+                 void* C, int ldC, cudaStream_t stream, DeviceState* st, bool own) {
   if (!st->pool) return fail(B200_EUNSUPPORTED, "the two-pass path needs the library's scratch pool");
   const long long ldx = (k + 7) & ~7;
+  const long long rows = two_pass_rows(m, k, own);
   void* xr = nullptr;
-  if (cudaError_t e = cudaMallocFromPoolAsync(&xr, static_cast<size_t>(m) * ldx * 2, st->pool, stream)) {  // stays in the pool until b200_shutdown
+  if (cudaError_t e = cudaMallocFromPoolAsync(&xr, static_cast<size_t>(rows) * ldx * 2, st->pool, stream)) {  // stays in the pool until b200_shutdown
     cudaGetLastError();
     if (e == cudaErrorMemoryAllocation) return kNoScratch;  // the caller decides: fused kernel, or an error for the explicit entry point
     return fail(B200_ECUDA, "cudaMallocFromPoolAsync: %s", cudaGetErrorString(e));
   }
   int rc = B200_OK;
-  for (int g = 0; rc == B200_OK && g < n / group_size; ++g) {  // stream order serialises the groups on the one XR buffer
-    rc = launch_xr<kB>(m, k, A, ldA, static_cast<const __half*>(R) + static_cast<long long>(g) * kB * ldR, ldR, xr, ldx, stream, st);
-    // row-major C[m][n] is the column-major (n x m, ld = ldC) result of  W_g . XR^T:  gemm_tn with the operands swapped
-    if (rc == B200_OK)
-      rc = b200_gemm_tn_f16(group_size, m, k, static_cast<const __half*>(B) + static_cast<long long>(g) * group_size * ldB, ldB, xr,
-                            static_cast<int>(ldx), static_cast<__half*>(C) + static_cast<long long>(g) * group_size, ldC, stream);
-  }
+  const bool whole_before = g_whole_k;
+  g_whole_k = whole_before || own;
+  for (int g = 0; rc == B200_OK && g < n / group_size; ++g)  // stream order serialises the groups and chunks on the one XR buffer
+    for (long long r0 = 0; rc == B200_OK && r0 < m; r0 += rows) {
+      const int mr = static_cast<int>(m - r0 < rows ? m - r0 : rows);
+      rc = launch_xr<kB>(mr, k, static_cast<const __half*>(A) + r0 * ldA, ldA, static_cast<const __half*>(R) + static_cast<long long>(g) * kB * ldR, ldR, xr,
+                         ldx, stream, st);
+      // row-major C[m][n] is the column-major (n x m, ld = ldC) result of  W_g . XR^T:  gemm_tn with the operands swapped
+      if (rc == B200_OK)
+        rc = b200_gemm_tn_f16(group_size, mr, k, static_cast<const __half*>(B) + static_cast<long long>(g) * group_size * ldB, ldB, xr,
+                              static_cast<int>(ldx), static_cast<__half*>(C) + r0 * ldC + static_cast<long long>(g) * group_size, ldC, stream);
+    }
+  g_whole_k = whole_before;
   const std::string keep = g_err;
   cudaFreeAsync(xr, stream);
   g_err = keep;
@@ -878,22 +913,47 @@ bool small_group_ok(int n, int group_size, int b) {
   return group_size == n || group_size % kBN == 0 || (group_size == 128 && kBN == 256 && b <= 64);
 }
 
-int choose_route(int m, int n, int group_size, int k, int b, const DeviceState* st) {
+// Whether small_kernel takes the OFT product: up to one 128 x 128 tile per SM always (see small_wins; 8 x 4096 x 4096 b 64
+// 35 -> 10 us), up to two as long as there is little to do (2000 tile steps, about 7 us) - it rotates X for each of its
+// narrow tiles - or M fits one tile
+// and W streams from memory.  Two tiles per SM, us against the best other route: 3332 x 896 x 464 b 16 14.6 / 16.9, 3967 x
+// 704 x 696 b 8 23.2 / 23.2, 3967 x 896 x 1472 b 8 31.8 / 25.2; M 17, N 22528, K 640 b 128 19.5 / 22.8; with unaligned rows of C 2802 x
+// 1453 x 776 b 8 27.3 / 28.1, 556 x 5034 x 3104 b 32 47.9 / 34.
+bool small_oft_wins(int m, int n, int k, int b, bool aligned, const DeviceState* st) {
+  const long long t128 = tiles_128(m, n);
+  const int steps = (k + 63) / 64;
+  if (t128 <= st->sm_count) return true;
+  if (t128 > 2ll * st->sm_count) return false;
+  return (aligned ? t128 * steps <= 2000 : steps <= 16) || (m <= 128 && (b < 128 || steps <= 32));
+}
+
+// aligned: rows of C start on 16-byte boundaries.
+int choose_route(int m, int n, int group_size, int k, int b, bool aligned, const DeviceState* st) {
   int path = g_oft_path != 0 ? g_oft_path : opt(kOptOftRoute);
   const bool can_share = kOftPair && st->pool != nullptr;  // routes 2, 3 and 4 need scratch from the pool
   if (path == 2 || path == 3 || path == 4 || path == 5) return can_share ? path : 1;
-  if (path == 1) return 1;
+  if (path == 1 || !can_share) return 1;
   const int plan_m = g_plan_m > 0 ? g_plan_m : m, plan_n = g_plan_n > 0 ? g_plan_n : n;
-  if (can_share && opt(kOptSmallTiles) != 0 && small_group_ok(n, group_size, b) && small_wins(plan_m, plan_n, st)) return 5;
-  const int min_tiles = b >= 128 ? 4 : 8;
-  if (!can_share || group_size < min_tiles * static_cast<int>(CurrCompParams::bN)) return 1;
+  if (opt(kOptSmallTiles) != 0 && small_group_ok(n, group_size, b) && small_oft_wins(plan_m, plan_n, k, b, aligned, st)) return 5;
+  const int k_steps = (k + 63) / 64, min_tiles = b >= 128 ? 4 : 8;
+  const bool wide = group_size >= min_tiles * static_cast<int>(CurrCompParams::bN);
+  // Rotation pass + plain GEMM (route 2).  Rows of C that are not 16-byte aligned and one group: the fused kernels store
+  // them a row at a time after a transpose in registers (route 1) or element by element (route 3); us on routes 1 / 2 / 3: 12375 x 1473 x
+  // 576 b 64 74.6 / 49.2 / 287, 2988 x 4253 x 4176 b 8 125 / 99 / 215, 39866 x 647 x 3456 b 128 254 / 260 / 298.  Short K, a wide
+  // group and more tiles than SM pairs: 16589 x 4904 x 384 b 128 114 / 82 / 140 (route 4 140), 6503 x 7008 x 512 b 64 68 / 56 / 86; with one
+  // round of tiles there is nothing to serialise the rotation with (647 x 4096 x 512 b 64 14.8 / 21.2 / 21.8).
+  if (g_more.n == 0) {
+    if (!aligned && group_size == n) return 2;
+    const long long t256 = ((static_cast<long long>(plan_m) + 255) / 256) * ((static_cast<long long>(group_size) + 255) / 256);
+    if (wide && k_steps < 16 && t256 > st->sm_count / 2) return 2;
+  }
+  if (!wide) return 1;
   if (g_more.n > 0) return 3;  // only oft3_kernel stores to further destinations
   // Route 4 also wants long tiles: its product pairs write C with the plain GEMM's epilogue (one 2-byte store per
   // element), which must fit beside a tile's MMAs.  Interleaved runs, route 4 / route 3 time: M 32768, N 28672, K 1024,
   // b 64: 1.61; M 262144, N 12288, K 2048, b 64 (3 pairs): 1.05; M 65536, N 28672, b 128 (2 pairs), K 2048: 0.86,
   // K 4096: 0.88.
   const RingPlan p = ring_plan(m, group_size, k, st);
-  const int k_steps = (k + 63) / 64;
   const bool split = p.rot_pairs >= 1 && p.rot_pairs <= 3 && k_steps >= 32 && (p.rot_pairs <= 2 || k_steps >= 64);
   return split ? 4 : 3;
 }
@@ -904,9 +964,10 @@ template <int kB>
 int launch_oft(int m, int n, int k, int group_size, const void* A, int ldA, const void* B, int ldB, const void* R, int ldR,
                void* C, int ldC, cudaStream_t stream, DeviceState* st) {
   constexpr int kBN = CurrCompParams::bN;
-  const int route = choose_route(m, n, group_size, k, kB, st);
+  const int route = choose_route(m, n, group_size, k, kB, (reinterpret_cast<uintptr_t>(C) & 15) == 0 && (ldC & 7) == 0, st);
   if (route == 2) {
-    const int rc = oft_two_pass<kB>(m, n, k, group_size, A, ldA, B, ldB, R, ldR, C, ldC, stream, st);
+    const bool own = g_oft_path != 2 && opt(kOptOftRoute) != 2;
+    const int rc = oft_two_pass<kB>(m, n, k, group_size, A, ldA, B, ldB, R, ldR, C, ldC, stream, st, own);
     if (rc != kNoScratch) return rc;
     if (g_oft_path == 2) return fail(B200_ECUDA, "no device memory for the %lld bytes of X.R scratch", static_cast<long long>(m) * ((k + 7) & ~7) * 2);
     // out of memory for X.R: the kernel that keeps X.R in tensor memory needs no scratch
@@ -1241,12 +1302,14 @@ int b200_oft_plan(int m, int n, int k, int group_size, int reconn_sz, int* path,
     return fail(B200_EINVAL, "bad plan arguments (m=%d n=%d k=%d group_size=%d reconn_sz=%d)", m, n, k, group_size, reconn_sz);
   DeviceState* st;
   if (int rc = device_state(&st)) return rc;
-  const int route = choose_route(m, n, group_size, k, reconn_sz == 8 ? 16 : reconn_sz, st);
+  const int route = choose_route(m, n, group_size, k, reconn_sz == 8 ? 16 : reconn_sz, n % 8 == 0, st);  // C packed and aligned
   // small_kernel forms X.R per tile of C on the chip and needs no scratch, like the kernel of route 1; a caller of the
   // plan sees the same 1 for both unless it asked for 5 itself
   if (path) *path = route == 5 && opt(kOptOftRoute) != 5 ? 1 : route;
   const int groups = n / group_size;
-  if (kernel_launches) *kernel_launches = (route == 2 ? 2 * groups : ((route == 3 || route == 4) ? groups : 1)) + (reconn_sz == 8 ? 1 : 0);
+  const long long rows = two_pass_rows(m, k, g_oft_path != 2 && opt(kOptOftRoute) != 2);
+  const int chunks = static_cast<int>((m + rows - 1) / rows);
+  if (kernel_launches) *kernel_launches = (route == 2 ? 2 * groups * chunks : ((route == 3 || route == 4) ? groups : 1)) + (reconn_sz == 8 ? 1 : 0);
   return B200_OK;
 }
 

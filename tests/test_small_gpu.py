@@ -127,3 +127,43 @@ def test_small_products_chained_on_two_streams(lib, cuda, pair_build):
     assert ops.device_status(lib)[0] == 0
     for b in (b1, b2, b3):
         assert torch.equal(b[6], want[6])
+
+
+@pytest.mark.parametrize("m,n,k,b,gs,want", [
+    (33000, 65, 4096, 64, None, 2),       # one group, unaligned rows: rotation pass in two chunks of X.R
+    (2300, 2300, 192, 64, None, 1),       # aligned (n % 4 == 0 but ldC padded to 8), short K, few N tiles
+    (2304, 2303, 448, 32, None, 2),       # unaligned, more than two 128 x 128 tiles per SM
+    (4400, 4104, 320, 8, None, 2),        # aligned, K below 1024 and more tiles than SM pairs
+    (2176, 2048, 136, 8, None, 1),        # two tiles per SM, little to do: the small-problem kernel
+    (4608, 4096, 576, 64, 2048, 2)])      # two wide groups
+def test_choice_between_the_routes_is_invisible(lib, cuda, pair_build, m, n, k, b, gs, want):
+    """Shapes either side of the lines between the small-problem kernel, the rotation pass + GEMM and the fused kernels:
+    the library's choice has the bits of the kernel that forms X.R per N tile, with aligned and unaligned rows of C."""
+    if not pair_build:
+        pytest.skip("the single-CTA build has one route")
+    import torch
+    from cute_mma_b200 import inputs
+
+    g = torch.Generator(device=cuda).manual_seed(94)
+    X = torch.randn((m, k), generator=g, device=cuda).half()
+    W = (torch.randn((n, k), generator=g, device=cuda) * 0.02).half()
+    groups = 1 if gs is None else n // gs
+    R = torch.from_numpy(inputs.pack_r(inputs.blocks_qr(groups, k // b, b, 94))).to(cuda)
+
+    def run(ldc, **opts):
+        C = torch.full((m + 1, ldc), -7.0, dtype=torch.float16, device=cuda)
+        import contextlib
+        with contextlib.ExitStack() as es:
+            for name, v in opts.items():
+                es.enter_context(ops.option(name, v, lib))
+            ops.oft_tn(m, n, k, X, k, W, k, R, k, C, ldc, group_size=gs, reconn_sz=b, lib=lib)
+        assert ops.device_status(lib)[0] == 0
+        assert bool((C[m] == -7.0).all()) and bool((C[:m, n:] == -7.0).all())
+        return C[:m, :n]
+
+    path = ops.oft_plan(m, n, k, group_size=gs, reconn_sz=b, lib=lib)["path"]
+    if n % 8 == 0 or want == 2:
+        assert path == {1: "fused_tmem", 2: "two_pass"}[want]
+    want_bits = run((n + 7) // 8 * 8, oft_route=1).contiguous().view(torch.int16)
+    for ldc in ((n + 7) // 8 * 8, n + (3 if n % 8 == 0 else 0)):
+        assert torch.equal(run(ldc).contiguous().view(torch.int16), want_bits), ldc
