@@ -106,6 +106,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
   cluster_sync_all();  // the pair's barriers exist before anything arrives on them from the other CTA
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();  // nothing above touches memory that an earlier kernel of the stream may still be writing
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (both CTAs)
@@ -159,6 +160,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__
         }
       }
       if (ok && args.tile_sync && done_rounds > 0) atomicAdd(args.rounds + rank, 1);
+      pdl_launch_dependents();  // all loads are on their way: the next kernel's launch may start under the last tile
     }
     __syncwarp();
   } else if (warp == 1) {

@@ -123,6 +123,7 @@ oft2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   cluster_sync_all();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();  // nothing above touches memory that an earlier kernel of the stream may still be writing
 
   if (warp == 0) {
     // -------------------------------------------------------------- producer of the {A, R} ring (both CTAs)
@@ -188,6 +189,7 @@ oft2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
         }
       }
       if (ok && args.tile_sync && done_rounds > 0) atomicAdd(args.rounds + 2 + rank, 1);
+      pdl_launch_dependents();  // all loads of W are on their way: the next kernel's launch may start under the last tile
     }
     __syncwarp();
   } else if (warp == 2) {

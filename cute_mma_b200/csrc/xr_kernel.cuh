@@ -84,6 +84,7 @@ xr_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CU
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();  // nothing above touches memory that an earlier kernel of the stream may still be writing
 
   if (warp == 0) {
     // -------------------------------------------------------------- producer
@@ -101,6 +102,7 @@ xr_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CU
           tma_load_2d(dst + T::kABytes, &tmap_r, full + 8 * s, k0 + su * T::kBK, 0);
         }
       }
+      pdl_launch_dependents();  // all loads are on their way
     }
     __syncwarp();
   } else if (warp == 1) {

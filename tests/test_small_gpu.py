@@ -167,3 +167,44 @@ def test_choice_between_the_routes_is_invisible(lib, cuda, pair_build, m, n, k, 
     want_bits = run((n + 7) // 8 * 8, oft_route=1).contiguous().view(torch.int16)
     for ldc in ((n + 7) // 8 * 8, n + (3 if n % 8 == 0 else 0)):
         assert torch.equal(run(ldc).contiguous().view(torch.int16), want_bits), ldc
+
+
+def test_dependent_launches_of_the_other_kernels(lib, cuda, pair_build):
+    """The same for the pair GEMM, the kernel that keeps X.R in tensor memory and the rotation pass: every product reads
+    what the last one wrote, and scratch from the pool is handed on between calls."""
+    if not pair_build:
+        pytest.skip("the pair kernels belong to the CTA-pair build")
+    import torch
+    from cute_mma_b200 import inputs
+
+    m, d, b = 1400, 2048, 64  # 11 x 16 tiles of 128 x 128
+    g = torch.Generator(device=cuda).manual_seed(96)
+    W = (torch.randn((d, d), generator=g, device=cuda) / 45).half()
+    R = torch.from_numpy(inputs.pack_r(inputs.blocks_qr(1, d // b, b, 96))).to(cuda)
+    x0 = torch.randn((m, d), generator=g, device=cuda).half()
+
+    def chain(bufs, stream, wait=False):
+        for i in range(6):
+            if i % 3 == 0:
+                ops.gemm_tn(d, m, d, W, d, bufs[i], d, bufs[i + 1], d, stream, lib=lib)
+            elif i % 3 == 1:
+                ops.oft_tn_two_pass(m, d, d, bufs[i], d, W, d, R, d, bufs[i + 1], d, stream, reconn_sz=b, lib=lib)
+            else:
+                ops.oft_tn_a_rw(m, d, d, bufs[i], d, W, d, R, d, bufs[i + 1], d, stream, reconn_sz=b, lib=lib)
+            ops.oft_tn(m, 768, d, bufs[i + 1], d, W, d, R, d, bufs[7 + i], 768, stream, reconn_sz=b, lib=lib)
+            if wait:
+                torch.cuda.synchronize()
+
+    new = lambda: [x0.clone()] + [torch.zeros_like(x0) for _ in range(6)] + [torch.zeros((m, 768), dtype=torch.float16, device=cuda) for _ in range(6)]
+    want = new()
+    chain(want, torch.cuda.current_stream(), wait=True)
+    s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+    b1, b2 = new(), new()
+    torch.cuda.synchronize()
+    for _ in range(3):
+        chain(b1, s1)
+        chain(b2, s2)
+    torch.cuda.synchronize()
+    assert ops.device_status(lib)[0] == 0
+    for got in (b1, b2):
+        assert all(torch.equal(x, y) for x, y in zip(got, want))
