@@ -935,18 +935,30 @@ bool small_group_ok(int n, int group_size, int b) {
   return group_size == n || group_size % kBN == 0 || (group_size == 128 && kBN == 256 && b <= 64);
 }
 
-// Whether small_kernel takes the OFT product: up to one 128 x 128 tile per SM always (see small_wins; 8 x 4096 x 4096 b 64
-// 35 -> 10 us), up to two as long as there is little to do (2000 tile steps, about 7 us) - it rotates X for each of its
-// narrow tiles - or M fits one tile
-// and W streams from memory.  Two tiles per SM, us against the best other route: 3332 x 896 x 464 b 16 14.6 / 16.9, 3967 x
-// 704 x 696 b 8 23.2 / 23.2, 3967 x 896 x 1472 b 8 31.8 / 25.2; M 17, N 22528, K 640 b 128 19.5 / 22.8; with unaligned rows of C 2802 x
-// 1453 x 776 b 8 27.3 / 28.1, 556 x 5034 x 3104 b 32 47.9 / 34.
+// Whether small_kernel takes the OFT product.  Up to one 128 x 128 tile per SM, and for M of one tile up to two, by a
+// model of its K loop: a step of a rotated tile costs 0.47 us (0.6 with 128 x 128 blocks; 0.66 for two CTAs of an SM),
+// a step of the other routes' 256 x 256 tiles 0.4 us on 74 pairs, plus fixed costs (rows of C that are not 16-byte aligned
+// cost the others 6 us more).  8 x 4096 x 4096 b 64 35 -> 10 us; 188 x 8320 x 3584 b 128, where K cannot be cut any more, 40 against 37.
+// Up to two tiles per SM otherwise only as long as there is little to do (2000 tile steps, about 7 us): it rotates X for
+// each of its narrow tiles.  us against the best other route: 3332 x 896 x 464 b 16 14.6 / 16.9, 3967 x 704 x 696 b 8 23.2 / 23.2, 3967 x
+// 896 x 1472 b 8 31.8 / 25.2; with unaligned rows of C 2802 x 1453 x 776 b 8 27.3 / 28.1, 556 x 5034 x 3104 b 32 47.9 / 34.
 bool small_oft_wins(int m, int n, int k, int b, bool aligned, const DeviceState* st) {
-  const long long t128 = tiles_128(m, n);
+  const long long t128 = tiles_128(m, n), pairs = st->sm_count / 2;
   const int steps = (k + 63) / 64;
-  if (t128 <= st->sm_count) return true;
   if (t128 > 2ll * st->sm_count) return false;
-  return (aligned ? t128 * steps <= 2000 : steps <= 16) || (m <= 128 && (b < 128 || steps <= 32));
+  if (t128 > st->sm_count && (aligned ? t128 * steps <= 2000 : steps <= 16)) return true;
+  if (t128 > st->sm_count && m > 128) return false;
+  const int tiles_x = (m + 127) / 128, n_tile = ((m + tiles_x - 1) / tiles_x + 15) / 16 * 16;
+  const int fixed = 2048 + (n_tile <= 64 ? 3 : 2) * n_tile * 128, stage = n_tile * 128 + b * 128 + 16384;  // as small_plan
+  const bool two = (113 * 1024 - fixed) / stage >= (b == 128 ? 4 : 3);
+  const long long slots = (two ? 2 : 1) * st->sm_count;
+  int split = 1;
+  while (steps >= 16 && split < 8 && t128 * (split + 1) <= slots && steps / (split + 1) >= 4) ++split;
+  const long long ctas = t128 * split, t256 = ((static_cast<long long>(m) + 255) / 256) * ((static_cast<long long>(n) + 255) / 256);
+  const double step = b == 128 ? 0.6 : (two && ctas > st->sm_count ? 0.66 : 0.47);
+  const double small = 6.0 + static_cast<double>((ctas + slots - 1) / slots) * steps / split * step;
+  const double other = (aligned ? 13.0 : 19.0) + 0.4 * static_cast<double>((t256 + pairs - 1) / pairs) * steps;
+  return small <= other;
 }
 
 // aligned: rows of C start on 16-byte boundaries.
