@@ -683,15 +683,16 @@ int launch_xr(int m, int k, const void* A, int ldA, const void* Rg, int ldR, voi
 
 constexpr int kNoScratch = -1000;  // internal: no device memory for X.R
 
-//
 // The library takes this route by itself (`own`) where the fused kernels are held up: rows of C that are not 16-byte
 // aligned, which the GEMM's epilogue stores along N whatever their alignment, and short K, where a ring kernel's
 // hand-off of X.R (about 2 us per row block) and its single accumulator show.  Then X.R is formed for at most
 // kOwnScratch bytes of rows at a time and the GEMM's K range is never cut, so that the bits are those of the routes
-// it stands in for.
+// it stands in for.  Not for K above 524288, where that scratch does not hold a row block of 256 rows.
 constexpr size_t kOwnScratch = size_t(256) << 20;
-long long two_pass_rows(int m, int k, bool own) {  // rows of X.R formed at a time
-  const size_t row_bytes = static_cast<size_t>((k + 7) & ~7) * 2;
+size_t xr_row_bytes(int k) { return ((static_cast<size_t>(k) + 7) & ~static_cast<size_t>(7)) * 2; }
+bool two_pass_fits(int k) { return xr_row_bytes(k) * 256 <= kOwnScratch; }
+long long two_pass_rows(int m, int k, bool own) {  // rows of X.R formed at a time; own: two_pass_fits(k)
+  const size_t row_bytes = xr_row_bytes(k);
   if (!own || static_cast<size_t>(m) * row_bytes <= kOwnScratch) return m;
   const long long most = static_cast<long long>(kOwnScratch / row_bytes) / 256 * 256, chunks = (m + most - 1) / most;
   return ((m + chunks - 1) / chunks + 255) / 256 * 256;  // equal chunks
@@ -977,7 +978,7 @@ int choose_route(int m, int n, int group_size, int k, int b, bool aligned, const
   // 576 b 64 74.6 / 49.2 / 287, 2988 x 4253 x 4176 b 8 125 / 99 / 215, 39866 x 647 x 3456 b 128 254 / 260 / 298.  Short K, a wide
   // group and more tiles than SM pairs: 16589 x 4904 x 384 b 128 114 / 82 / 140 (route 4 140), 6503 x 7008 x 512 b 64 68 / 56 / 86; with one
   // round of tiles there is nothing to serialise the rotation with (647 x 4096 x 512 b 64 14.8 / 21.2 / 21.8).
-  if (g_more.n == 0) {
+  if (g_more.n == 0 && two_pass_fits(k)) {
     if (!aligned && group_size == n) return 2;
     const long long t256 = ((static_cast<long long>(plan_m) + 255) / 256) * ((static_cast<long long>(group_size) + 255) / 256);
     if (wide && k_steps < 16 && t256 > st->sm_count / 2) return 2;
@@ -1342,9 +1343,12 @@ int b200_oft_plan(int m, int n, int k, int group_size, int reconn_sz, int* path,
   // plan sees the same 1 for both unless it asked for 5 itself
   if (path) *path = route == 5 && opt(kOptOftRoute) != 5 ? 1 : route;
   const int groups = n / group_size;
-  const long long rows = two_pass_rows(m, k, g_oft_path != 2 && opt(kOptOftRoute) != 2);
-  const int chunks = static_cast<int>((m + rows - 1) / rows);
-  if (kernel_launches) *kernel_launches = (route == 2 ? 2 * groups * chunks : ((route == 3 || route == 4) ? groups : 1)) + (reconn_sz == 8 ? 1 : 0);
+  int launches = route == 3 || route == 4 ? groups : 1;
+  if (route == 2) {
+    const long long rows = two_pass_rows(m, k, opt(kOptOftRoute) != 2);
+    launches = 2 * groups * static_cast<int>((m + rows - 1) / rows);
+  }
+  if (kernel_launches) *kernel_launches = launches + (reconn_sz == 8 ? 1 : 0);
   return B200_OK;
 }
 

@@ -208,3 +208,32 @@ def test_dependent_launches_of_the_other_kernels(lib, cuda, pair_build):
     assert ops.device_status(lib)[0] == 0
     for got in (b1, b2):
         assert all(torch.equal(x, y) for x, y in zip(got, want))
+
+
+def test_rows_of_x_longer_than_a_megabyte(lib, cuda, pair_build):
+    """K above 524288: the plan answers, and a call with unaligned rows of C has the bits of the kernel that forms X.R
+    per N tile."""
+    import torch
+
+    b, k = 64, 524288 + 64
+    assert ops.oft_plan(4096, 256, k, reconn_sz=b, lib=lib)["path"] in ("fused_tmem", "fused_ring")
+    assert ops.oft_plan(4096, 4096, k, reconn_sz=b, lib=lib)["kernel_launches"] >= 1
+    if not pair_build:
+        return
+    m, n = 300, 257
+    g = torch.Generator(device=cuda).manual_seed(98)
+    X = torch.randn((m, k), generator=g, device=cuda).half()
+    W = (torch.randn((n, k), generator=g, device=cuda) * 0.02).half()
+    R = (torch.randn((b, k), generator=g, device=cuda) * 0.1).half()
+
+    def run(**opts):
+        import contextlib
+        C = torch.full((m + 1, n), -7.0, dtype=torch.float16, device=cuda)
+        with contextlib.ExitStack() as es:
+            for name, v in opts.items():
+                es.enter_context(ops.option(name, v, lib))
+            ops.oft_tn(m, n, k, X, k, W, k, R, k, C, n, reconn_sz=b, lib=lib)
+        assert ops.device_status(lib)[0] == 0
+        return C.view(torch.int16)
+
+    assert torch.equal(run(small_tiles=0), run(oft_route=1))
