@@ -302,13 +302,16 @@ int launch_gemm_bn(int m, int n, int k, const void* A, int ldA, const void* B, i
                    int k2, const void* A2, int ldA2, const void* B2, int ldB2, float alpha, float beta);
 
 // ---- small problems: small_kernel ----------------------------------------------------------------------
-// Sizes that decide between the kernels (and how often K is cut) in the place of a call's own: an entry point that
-// computes one product in parts (row chunks, slabs of N) sets them to the whole product's, so that the parts have the
-// bits of a single call.
-thread_local int g_plan_m = 0, g_plan_n = 0;
-struct PlanAs {
-  PlanAs(int m, int n) { g_plan_m = m; g_plan_n = n; }
-  ~PlanAs() { g_plan_m = g_plan_n = 0; }
+// The whole product of which a call computes a part (row chunks, slabs of N, pieces of both).  Whether and how often K
+// is cut follows the whole's sizes, so that the parts have the bits of a single call; zeros: the call is the whole.
+struct Whole {
+  int m = 0, n = 0, group_size = 0;
+};
+thread_local Whole g_whole;
+struct PartOf {
+  const Whole before = g_whole;
+  PartOf(int m, int n, int group_size) { g_whole.m = m; g_whole.n = n; g_whole.group_size = group_size; }
+  ~PartOf() { g_whole = before; }
 };
 // Tiles of 128 x 128 of an m x n result.
 long long tiles_128(int m, int n) { return ((static_cast<long long>(m) + 127) / 128) * ((static_cast<long long>(n) + 127) / 128); }
@@ -334,60 +337,72 @@ bool small_wins(int m, int n, int steps, const DeviceState* st) {
   return small < pair;
 }
 
-struct SmallPlan {
-  int tiles_m, tiles_n, n_tile, split, stages, xbufs, smem;
+// What the geometry of a launch depends on beside the sizes: an instance of small_kernel.
+struct SmallKind {
+  int bk, gran, unit, r_bytes, min_stages, tail_bytes, max_stages;
+  bool rot;
 };
-// Geometry for P [m][k], Q [n][k]; b > 0: Q is rotated by b x b blocks.
 template <class T>
-SmallPlan small_plan(int m, int n, int k, const DeviceState* st) {
-  constexpr int gran = T::kMn ? T::kChunk : 16, unit = T::kB == 128 ? 2 : 1;
-  constexpr int min_stages = T::kB == 128 ? 4 : 3;  // both steps of a 128 x 128 block, and the next block's behind them
-  constexpr int half_sm = 113 * 1024, whole_sm = 232448;
-  const int steps = (k + T::kBK * unit - 1) / (T::kBK * unit) * unit;
-  struct Ring { int n_tile, xbufs, stage, fixed, stages; bool two; };
-  auto ring = [&](int rows) {  // for a Q of this many rows
-    Ring r;
-    const int tiles = (rows + 127) / 128;
-    r.n_tile = ((rows + tiles - 1) / tiles + gran - 1) / gran * gran;
-    r.xbufs = T::kRot ? (r.n_tile <= 64 ? 3 : 2) : 0;
-    r.stage = r.n_tile * 128 + T::kRBytes + T::kPBytes;
-    r.fixed = 1024 + r.xbufs * r.n_tile * 128 + T::kTailBytes;
-    r.stages = (half_sm - r.fixed) / r.stage;
-    r.two = r.stages >= min_stages;  // two CTAs per SM
-    if (!r.two) r.stages = (whole_sm - r.fixed) / r.stage;
-    return r;
-  };
-  Ring r = ring(n);
-  // As many pieces along K as there is room for CTAs at once; at least four K steps each, and none below 16 steps (a
-  // K loop of 16 steps takes about 4 us, adding up the pieces 1.5).
-  const long long tiles = g_plan_m > 0 ? tiles_128(g_plan_m, g_plan_n) : tiles_128(m, n);
-  const long long slots = (ring(g_plan_m > 0 ? g_plan_m : n).two ? 2 : 1) * st->sm_count;
+constexpr SmallKind small_kind() {
+  // 128 x 128 blocks: both steps of a block, and the next block's behind them
+  return {T::kBK, T::kMn ? T::kChunk : 16, T::kB == 128 ? 2 : 1, T::kRBytes, T::kB == 128 ? 4 : 3, T::kTailBytes, T::kMaxStages, T::kRot};
+}
+SmallKind small_oft_kind(int b) {
+  switch (b) {
+    case 32: return small_kind<SmallTraits<__half, __half, false, 32>>();
+    case 64: return small_kind<SmallTraits<__half, __half, false, 64>>();
+    case 128: return small_kind<SmallTraits<__half, __half, false, 128>>();
+    default: return small_kind<SmallTraits<__half, __half, false, 16>>();
+  }
+}
+
+struct SmallPlan {
+  int steps, n_tile, xbufs, stage_bytes, fixed_bytes, stages, smem;
+  bool two;              // two CTAs per SM
+  long long slots;       // CTAs resident at once
+};
+constexpr int kWholeSmBytes = 232448;
+// Geometry for P [m][k], Q [n][k] (rotated if the kind says so), K in one piece.
+SmallPlan small_plan(const SmallKind& kind, int m, int n, int k, const DeviceState* st) {
+  constexpr int half_sm = 113 * 1024;
   SmallPlan p;
-  p.split = 1;
-  if (steps >= 16)
-    while (p.split < 8 && tiles * (p.split + 1) <= slots && steps / (p.split + 1) >= 4) ++p.split;
-  if (opt(kOptSmallSplit) >= 1 && opt(kOptSmallSplit) <= 8) p.split = opt(kOptSmallSplit);
-  if (opt(kOptGemmSplit) == 0) p.split = 1;
-  if (p.split > steps / unit) p.split = steps / unit;
-  if (opt(kOptSmallStages) >= 2) r.stages = opt(kOptSmallStages);
-  if (r.stages > (whole_sm - r.fixed) / r.stage) r.stages = (whole_sm - r.fixed) / r.stage;
-  if (r.stages < min_stages) r.stages = min_stages;
-  if (r.stages > T::kMaxStages) r.stages = T::kMaxStages;
-  p.tiles_m = (m + 127) / 128;
-  p.tiles_n = (n + 127) / 128;
-  p.n_tile = r.n_tile;
-  p.xbufs = r.xbufs;
-  p.stages = r.stages;
-  p.smem = r.fixed + r.stages * r.stage;
+  p.steps = (k + kind.bk * kind.unit - 1) / (kind.bk * kind.unit) * kind.unit;
+  const int tiles_n = (n + 127) / 128;
+  p.n_tile = ((n + tiles_n - 1) / tiles_n + kind.gran - 1) / kind.gran * kind.gran;
+  p.xbufs = kind.rot ? (p.n_tile <= 64 ? 3 : 2) : 0;
+  p.stage_bytes = p.n_tile * 128 + kind.r_bytes + 128 * 128;
+  p.fixed_bytes = 1024 + p.xbufs * p.n_tile * 128 + kind.tail_bytes;
+  p.stages = (half_sm - p.fixed_bytes) / p.stage_bytes;
+  p.two = p.stages >= kind.min_stages;
+  if (!p.two) p.stages = (kWholeSmBytes - p.fixed_bytes) / p.stage_bytes;
+  p.slots = (p.two ? 2 : 1) * st->sm_count;
+  if (opt(kOptSmallStages) >= 2) p.stages = opt(kOptSmallStages);
+  if (p.stages > (kWholeSmBytes - p.fixed_bytes) / p.stage_bytes) p.stages = (kWholeSmBytes - p.fixed_bytes) / p.stage_bytes;
+  if (p.stages < kind.min_stages) p.stages = kind.min_stages;
+  if (p.stages > kind.max_stages) p.stages = kind.max_stages;
+  p.smem = p.fixed_bytes + p.stages * p.stage_bytes;
   if (p.smem < 78 * 1024) p.smem = 78 * 1024;  // at most two CTAs of an SM: their tensor memory (256 columns each) is all there is
   return p;
 }
+// Pieces along K of an m x n product: as many as there is room for CTAs at once; at least four K steps each, and none
+// below 16 steps (a K loop of 16 steps takes about 4 us, adding up the pieces 1.5).
+int small_pieces(const SmallKind& kind, int m, int n, int k, const DeviceState* st) {
+  const SmallPlan p = small_plan(kind, m, n, k, st);
+  const long long tiles = tiles_128(m, n);
+  int split = 1;
+  if (p.steps >= 16)
+    while (split < 8 && tiles * (split + 1) <= p.slots && p.steps / (split + 1) >= 4) ++split;
+  if (opt(kOptSmallSplit) >= 1 && opt(kOptSmallSplit) <= 8) split = opt(kOptSmallSplit);
+  if (opt(kOptGemmSplit) == 0) split = 1;
+  return split < p.steps / kind.unit ? split : p.steps / kind.unit;
+}
 
 template <class T>
-int launch_small(const SmallPlan& p, int m, int n, int k, const void* P, int ldP, const char* p_name, const void* Q, int ldQ, const char* q_name,
+int launch_small(int split, int m, int n, int k, const void* P, int ldP, const char* p_name, const void* Q, int ldQ, const char* q_name,
                  const void* R, int ldR, int group_size, void* C, int ldC, float alpha, float beta, cudaStream_t stream, DeviceState* st) {
   using TIn = typename T::TIn;
   using TOut = typename T::TOut;
+  const SmallPlan p = small_plan(small_kind<T>(), m, n, k, st);
   CUtensorMap mp, mq, mr;
   int p3d = 0, q3d = 0;
   if constexpr (!T::kMn) {
@@ -406,11 +421,12 @@ int launch_small(const SmallPlan& p, int m, int n, int k, const void* P, int ldP
     mr = mq;  // never read
   }
   const int vec = (reinterpret_cast<uintptr_t>(C) % (4 * sizeof(TOut))) == 0 && ldC % 4 == 0;
-  SmallArgs args{m, n, k, C, ldC, st->status, p.n_tile, p.tiles_n, p.split, p.stages, p.xbufs, group_size, p3d, q3d, vec, alpha, beta};
+  const int tiles_m = (m + 127) / 128, tiles_n = (n + 127) / 128;
+  SmallArgs args{m, n, k, C, ldC, st->status, p.n_tile, tiles_n, split, p.stages, p.xbufs, group_size, p3d, q3d, vec, alpha, beta};
   auto kernel = small_kernel<T>;
-  if (int rc = opt_in_smem(kernel, 232448)) return rc;
+  if (int rc = opt_in_smem(kernel, kWholeSmBytes)) return rc;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(static_cast<unsigned>(p.tiles_m * p.tiles_n * p.split));
+  cfg.gridDim = dim3(static_cast<unsigned>(tiles_m * tiles_n * split));
   cfg.blockDim = dim3(T::kThreads);
   cfg.dynamicSmemBytes = static_cast<size_t>(p.smem);
   cfg.stream = stream;
@@ -418,10 +434,10 @@ int launch_small(const SmallPlan& p, int m, int n, int k, const void* P, int ldP
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = opt(kOptPdl) != 0 ? 1 : 0;
   attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = static_cast<unsigned>(p.split);
+  attr[1].val.clusterDim.x = static_cast<unsigned>(split);
   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = p.split > 1 ? 2 : 1;
+  cfg.numAttrs = split > 1 ? 2 : 1;
   CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, mp, mq, mr, args));
   return B200_OK;
 }
@@ -460,7 +476,7 @@ int launch_gemm_bn(int m, int n, int k, const void* A, int ldA, const void* B, i
   if constexpr (kPair) {
     if (k2 == 0 && !g_whole_k && (opt(kOptSmallTiles) < 0 ? small_wins(m, n, (k + T1::kBK - 1) / T1::kBK, st) : opt(kOptSmallTiles) != 0)) {
       using TS = SmallTraits<TIn, TOut, kNT, 0>;
-      return launch_small<TS>(small_plan<TS>(m, n, k, st), m, n, k, A, ldA, "A", B, ldB, "B", nullptr, 0, 1, C, ldC, alpha, beta, stream, st);
+      return launch_small<TS>(small_pieces(small_kind<TS>(), m, n, k, st), m, n, k, A, ldA, "A", B, ldB, "B", nullptr, 0, 1, C, ldC, alpha, beta, stream, st);
     }
   }
   constexpr int kBoxN = kPair ? T2::kBNHalf : T1::kBN;
@@ -944,33 +960,38 @@ bool small_group_ok(int n, int group_size, int b) {
 // Up to two tiles per SM otherwise only as long as there is little to do (2000 tile steps, about 7 us): it rotates X for
 // each of its narrow tiles.  us against the best other route: 3332 x 896 x 464 b 16 14.6 / 16.9, 3967 x 704 x 696 b 8 23.2 / 23.2, 3967 x
 // 896 x 1472 b 8 31.8 / 25.2; with unaligned rows of C 2802 x 1453 x 776 b 8 27.3 / 28.1, 556 x 5034 x 3104 b 32 47.9 / 34.
-bool small_oft_wins(int m, int n, int k, int b, bool aligned, const DeviceState* st) {
+bool small_oft_wins(int m, int n, int k, int b, int pieces, bool aligned, const DeviceState* st) {
   const long long t128 = tiles_128(m, n), pairs = st->sm_count / 2;
   const int steps = (k + 63) / 64;
   if (t128 > 2ll * st->sm_count) return false;
   if (t128 > st->sm_count && (aligned ? t128 * steps <= 2000 : steps <= 16)) return true;
   if (t128 > st->sm_count && m > 128) return false;
-  const int tiles_x = (m + 127) / 128, n_tile = ((m + tiles_x - 1) / tiles_x + 15) / 16 * 16;
-  const int fixed = 2048 + (n_tile <= 64 ? 3 : 2) * n_tile * 128, stage = n_tile * 128 + b * 128 + 16384;  // as small_plan
-  const bool two = (113 * 1024 - fixed) / stage >= (b == 128 ? 4 : 3);
-  const long long slots = (two ? 2 : 1) * st->sm_count;
-  int split = 1;
-  while (steps >= 16 && split < 8 && t128 * (split + 1) <= slots && steps / (split + 1) >= 4) ++split;
-  const long long ctas = t128 * split, t256 = ((static_cast<long long>(m) + 255) / 256) * ((static_cast<long long>(n) + 255) / 256);
-  const double step = b == 128 ? 0.6 : (two && ctas > st->sm_count ? 0.66 : 0.47);
-  const double small = 6.0 + static_cast<double>((ctas + slots - 1) / slots) * steps / split * step;
+  const SmallPlan p = small_plan(small_oft_kind(b), n, m, k, st);
+  const long long ctas = t128 * pieces, t256 = ((static_cast<long long>(m) + 255) / 256) * ((static_cast<long long>(n) + 255) / 256);
+  const double step = b == 128 ? 0.6 : (p.two && ctas > st->sm_count ? 0.66 : 0.47);
+  const double small = 6.0 + static_cast<double>((ctas + p.slots - 1) / p.slots) * steps / pieces * step;
   const double other = (aligned ? 13.0 : 19.0) + 0.4 * static_cast<double>((t256 + pairs - 1) / pairs) * steps;
   return small <= other;
 }
 
-// aligned: rows of C start on 16-byte boundaries.
-int choose_route(int m, int n, int group_size, int k, int b, bool aligned, const DeviceState* st) {
+// Whether small_kernel takes the product, and in how many pieces of K.  Cut products are decided by the whole's sizes
+// alone (not by where a part's C lies, and not for a slab that is one small group by itself of a whole whose groups the
+// kernel cannot take); with K whole, the kernel has the bits of every other route and each part may choose for itself.
+bool oft_takes_small(const Whole& w, int m, int n, int group_size, int k, int b, bool aligned, const DeviceState* st, int* pieces) {
+  *pieces = small_group_ok(w.n, w.group_size, b) ? small_pieces(small_oft_kind(b), w.n, w.m, k, st) : 1;
+  if (*pieces > 1) return small_oft_wins(w.m, w.n, k, b, *pieces, true, st);
+  return small_group_ok(n, group_size, b) && small_oft_wins(m, n, k, b, 1, aligned, st);
+}
+
+// aligned: rows of C start on 16-byte boundaries.  *pieces: those of K on route 5.
+int choose_route(int m, int n, int group_size, int k, int b, bool aligned, const DeviceState* st, int* pieces) {
   int path = g_oft_path != 0 ? g_oft_path : opt(kOptOftRoute);
   const bool can_share = kOftPair && st->pool != nullptr;  // routes 2, 3 and 4 need scratch from the pool
+  const Whole w = g_whole.m > 0 ? g_whole : Whole{m, n, group_size};
+  *pieces = path == 5 && small_group_ok(w.n, w.group_size, b) ? small_pieces(small_oft_kind(b), w.n, w.m, k, st) : 1;
   if (path == 2 || path == 3 || path == 4 || path == 5) return can_share ? path : 1;
   if (path == 1 || !can_share) return 1;
-  const int plan_m = g_plan_m > 0 ? g_plan_m : m, plan_n = g_plan_n > 0 ? g_plan_n : n;
-  if (opt(kOptSmallTiles) != 0 && small_group_ok(n, group_size, b) && small_oft_wins(plan_m, plan_n, k, b, aligned, st)) return 5;
+  if (opt(kOptSmallTiles) != 0 && oft_takes_small(w, m, n, group_size, k, b, aligned, st, pieces)) return 5;
   const int k_steps = (k + 63) / 64, min_tiles = b >= 128 ? 4 : 8;
   const bool wide = group_size >= min_tiles * static_cast<int>(CurrCompParams::bN);
   // Rotation pass + plain GEMM (route 2).  Rows of C that are not 16-byte aligned and one group: the fused kernels store
@@ -980,7 +1001,7 @@ int choose_route(int m, int n, int group_size, int k, int b, bool aligned, const
   // round of tiles there is nothing to serialise the rotation with (647 x 4096 x 512 b 64 14.8 / 21.2 / 21.8).
   if (g_more.n == 0 && two_pass_fits(k)) {
     if (!aligned && group_size == n) return 2;
-    const long long t256 = ((static_cast<long long>(plan_m) + 255) / 256) * ((static_cast<long long>(group_size) + 255) / 256);
+    const long long t256 = ((static_cast<long long>(m) + 255) / 256) * ((static_cast<long long>(group_size) + 255) / 256);
     if (wide && k_steps < 16 && t256 > st->sm_count / 2) return 2;
   }
   if (!wide) return 1;
@@ -1000,7 +1021,8 @@ template <int kB>
 int launch_oft(int m, int n, int k, int group_size, const void* A, int ldA, const void* B, int ldB, const void* R, int ldR,
                void* C, int ldC, cudaStream_t stream, DeviceState* st) {
   constexpr int kBN = CurrCompParams::bN;
-  const int route = choose_route(m, n, group_size, k, kB, (reinterpret_cast<uintptr_t>(C) & 15) == 0 && (ldC & 7) == 0, st);
+  int pieces = 1;
+  const int route = choose_route(m, n, group_size, k, kB, (reinterpret_cast<uintptr_t>(C) & 15) == 0 && (ldC & 7) == 0, st, &pieces);
   if (route == 2) {
     const bool own = g_oft_path != 2 && opt(kOptOftRoute) != 2;
     const int rc = oft_two_pass<kB>(m, n, k, group_size, A, ldA, B, ldB, R, ldR, C, ldC, stream, st, own);
@@ -1011,7 +1033,7 @@ int launch_oft(int m, int n, int k, int group_size, const void* A, int ldA, cons
   if constexpr (kOftPair) {
     if (route == 5 && small_group_ok(n, group_size, kB)) {
       using TS = SmallTraits<__half, __half, false, kB>;
-      return launch_small<TS>(small_plan<TS>(n, m, k, st), n, m, k, B, ldB, "B", A, ldA, "A", R, ldR, group_size, C, ldC, 1.f, 0.f, stream, st);
+      return launch_small<TS>(pieces, n, m, k, B, ldB, "B", A, ldA, "A", R, ldR, group_size, C, ldC, 1.f, 0.f, stream, st);
     }
     if ((route == 3 || route == 4) && (group_size == n || group_size % kBN == 0)) {
       const int rc = oft_ring<kB>(m, n, k, group_size, A, ldA, B, ldB, R, ldR, C, ldC, stream, st, route == 4);
@@ -1226,6 +1248,27 @@ int oft_dispatch(int m, int n, int k, int group_size, int b, const void* A, int 
   }
 }
 
+// The product stored to n_dst buffers.
+int oft_gather(int m, int n, int k, int group_size, int b, const void* A, int ldA, const void* B, int ldB, const void* R, int ldR, int n_dst,
+               void* const* C_dst, int ldC, cudaStream_t stream) {
+  g_err.clear();
+  if (n_dst < 1 || n_dst > 8 || !C_dst) return fail(B200_EINVAL, "n_dst=%d: between 1 and 8 destinations", n_dst);
+  for (int d = 0; d < n_dst; ++d)
+    if (!C_dst[d] && m > 0 && n > 0) return fail(B200_EINVAL, "destination %d is null", d);
+  g_more = MoreDst{};
+  g_more.n = n_dst - 1;
+  for (int d = 1; d < n_dst; ++d) g_more.p[d - 1] = static_cast<__half*>(C_dst[d]);
+  int rc = oft_dispatch(m, n, k, group_size, b, A, ldA, B, ldB, R, ldR, C_dst[0], ldC, stream);
+  const bool stored = g_more.stored;
+  g_more = MoreDst{};
+  if (rc != B200_OK || stored || m == 0 || n == 0) return rc;
+  // a route without the multi-destination epilogue (few N tiles per group, k = 0, no scratch): copy the result
+  for (int d = 1; d < n_dst; ++d)
+    CUDA_TRY(cudaMemcpy2DAsync(C_dst[d], static_cast<size_t>(ldC) * 2, C_dst[0], static_cast<size_t>(ldC) * 2, static_cast<size_t>(n) * 2, m,
+                               cudaMemcpyDeviceToDevice, stream));
+  return B200_OK;
+}
+
 int stage_reserve(DeviceState* st, int slot, size_t bytes) {
   if (st->stage_bytes[slot] >= bytes) return B200_OK;
   if (st->stage[slot]) CUDA_TRY(cudaFree(st->stage[slot]));
@@ -1338,7 +1381,8 @@ int b200_oft_plan(int m, int n, int k, int group_size, int reconn_sz, int* path,
     return fail(B200_EINVAL, "bad plan arguments (m=%d n=%d k=%d group_size=%d reconn_sz=%d)", m, n, k, group_size, reconn_sz);
   DeviceState* st;
   if (int rc = device_state(&st)) return rc;
-  const int route = choose_route(m, n, group_size, k, reconn_sz == 8 ? 16 : reconn_sz, n % 8 == 0, st);  // C packed and aligned
+  int pieces = 1;
+  const int route = choose_route(m, n, group_size, k, reconn_sz == 8 ? 16 : reconn_sz, n % 8 == 0, st, &pieces);  // C packed and aligned
   // small_kernel forms X.R per tile of C on the chip and needs no scratch, like the kernel of route 1; a caller of the
   // plan sees the same 1 for both unless it asked for 5 itself
   if (path) *path = route == 5 && opt(kOptOftRoute) != 5 ? 1 : route;
@@ -1383,8 +1427,9 @@ int b200_oft_tn_f16_host(int m, int n, int k, int group_size, int reconn_sz, con
   // Rows of X go up, are multiplied and come back chunk by chunk on three streams, so that the upload of chunk
   // i + 1, the product of chunk i and the download of chunk i - 1 overlap (the link is full duplex and the
   // download of Y is the longest leg: 3.76 GB against 1.55 GB up at M 65536, K 8192, N 28672).  Results do not
-  // depend on the chunking: an element of Y only ever sees its own row of X and its own column of W.
-  const PlanAs whole(m, n);
+  // depend on the chunking: an element of Y only ever sees its own row of X and its own column of W, and K is cut as
+  // for the whole product.
+  const PartOf whole(m, n, group_size);
   constexpr int kMaxChunks = 16;
   int chunk_rows = ((m + kMaxChunks - 1) / kMaxChunks + 255) & ~255;
   if (chunk_rows < 2048) chunk_rows = 2048;
@@ -1603,7 +1648,7 @@ int b200_oft_tn_f16_sharded(int m, int n, int k, int group_size, int reconn_sz, 
   int cur = 0;
   CUDA_TRY(cudaGetDevice(&cur));
   int rc = B200_OK;
-  const PlanAs whole(m, n);
+  const PartOf whole(m, n, group_size);
   for (int r = 0; rc == B200_OK && r < world; ++r) {
     int n0 = 0, n1 = 0;
     rc = b200_shard_range(n, group_size, world, r, &n0, &n1);
@@ -1625,23 +1670,19 @@ int b200_oft_tn_f16_sharded(int m, int n, int k, int group_size, int reconn_sz, 
 
 int b200_oft_tn_f16_gather(int m, int n, int k, int group_size, int reconn_sz, const void* A, int ldA, const void* B, int ldB,
                            const void* R, int ldR, int n_dst, void* const* C_dst, int ldC, void* stream_v) {
+  return oft_gather(m, n, k, group_size, reconn_sz, A, ldA, B, ldB, R, ldR, n_dst, C_dst, ldC, static_cast<cudaStream_t>(stream_v));
+}
+
+int b200_oft_tn_f16_part(int whole_m, int whole_n, int whole_group_size, int m, int n, int k, int group_size, int reconn_sz, const void* A, int ldA,
+                         const void* B, int ldB, const void* R, int ldR, int n_dst, void* const* C_dst, int ldC, void* stream_v) {
   g_err.clear();
-  if (n_dst < 1 || n_dst > 8 || !C_dst) return fail(B200_EINVAL, "n_dst=%d: between 1 and 8 destinations", n_dst);
-  for (int d = 0; d < n_dst; ++d)
-    if (!C_dst[d] && m > 0 && n > 0) return fail(B200_EINVAL, "destination %d is null", d);
-  cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
-  g_more = MoreDst{};
-  g_more.n = n_dst - 1;
-  for (int d = 1; d < n_dst; ++d) g_more.p[d - 1] = static_cast<__half*>(C_dst[d]);
-  int rc = oft_dispatch(m, n, k, group_size, reconn_sz, A, ldA, B, ldB, R, ldR, C_dst[0], ldC, stream);
-  const bool stored = g_more.stored;
-  g_more = MoreDst{};
-  if (rc != B200_OK || stored || m == 0 || n == 0) return rc;
-  // a route without the multi-destination epilogue (few N tiles per group, k = 0, no scratch): copy the result
-  for (int d = 1; d < n_dst; ++d)
-    CUDA_TRY(cudaMemcpy2DAsync(C_dst[d], static_cast<size_t>(ldC) * 2, C_dst[0], static_cast<size_t>(ldC) * 2, static_cast<size_t>(n) * 2, m,
-                               cudaMemcpyDeviceToDevice, stream));
-  return B200_OK;
+  if (whole_m <= 0 || whole_n <= 0 || whole_group_size <= 0 || whole_n % whole_group_size != 0 || n > whole_n)
+    return fail(B200_EINVAL, "bad whole of a part (whole_m=%d whole_n=%d whole_group_size=%d n=%d)", whole_m, whole_n, whole_group_size, n);
+  if (group_size != whole_group_size && !(whole_group_size == whole_n && group_size == n))
+    return fail(B200_EINVAL, "group_size=%d: a part has its whole's groups (%d), or is one group of its own width where the whole is one", group_size,
+                whole_group_size);
+  const PartOf whole(whole_m, whole_n, whole_group_size);
+  return oft_gather(m, n, k, group_size, reconn_sz, A, ldA, B, ldB, R, ldR, n_dst, C_dst, ldC, static_cast<cudaStream_t>(stream_v));
 }
 
 int b200_tile_coord(unsigned tiles_m, unsigned tiles_n, unsigned idx, unsigned* tile_m, unsigned* tile_n) {

@@ -25,18 +25,18 @@ def oft_tn_slab(m, n_total, k, A, ldA, B_slab, ldB, R_slab, ldR, C_slab, ldC, n0
 
     B_slab points at row n0 of B (or at a private [n1-n0][k] copy), C_slab at column n0 of C (ldC = n_total)
     or at a private [m][n1-n0] buffer (ldC = n1-n0).  R_slab points at the first stored R row of the
-    slab's first group.  ``compute`` (default: the CUDA kernel) exists so that the partition logic can be
-    exercised on CPU ranks."""
+    slab's first group.  The slab has the bits of one oft_tn over all n_total columns.  ``compute`` (default: the
+    CUDA kernel) exists so that the partition logic can be exercised on CPU ranks."""
     n_loc = n1 - n0
     if n_loc <= 0:
         return
     gs = n_total if group_size is None else group_size
     gs_loc = n_loc if gs >= n_total else gs   # a single group spans the whole slab
-    fn = compute or ops.oft_tn
-    kwargs = dict(group_size=gs_loc, reconn_sz=reconn_sz)
     if compute is None:
-        kwargs["lib"] = lib
-    fn(m, n_loc, k, A, ldA, B_slab, ldB, R_slab, ldR, C_slab, ldC, stream, **kwargs)
+        ops.oft_tn_part((m, n_total, min(gs, n_total)), m, n_loc, k, A, ldA, B_slab, ldB, R_slab, ldR, [C_slab], ldC, stream,
+                        group_size=gs_loc, reconn_sz=reconn_sz, lib=lib)
+    else:
+        compute(m, n_loc, k, A, ldA, B_slab, ldB, R_slab, ldR, C_slab, ldC, stream, group_size=gs_loc, reconn_sz=reconn_sz)
 
 
 def all_gather_c(c_local, world: int | None = None):
@@ -69,7 +69,8 @@ class HostSlabRunner:
     rank is gathered, the rank's slab product runs on those world x chunk rows and their [rows][n_loc] piece of Y
     goes back to host memory while later chunks are still uploading, gathering and multiplying (four streams:
     upload, collective, product, download).  The slab of W^T and R go up right behind the first chunk of X.
-    Device buffers are allocated once per runner; rows are independent, so the chunking changes no bit.
+    Device buffers are allocated once per runner; every chunk has the bits of one oft_tn over all rows and columns
+    (ops.oft_tn_part), so the chunking changes no bit.
     ``compute`` / ``device`` exist so that the data movement can be exercised on CPU ranks over gloo with the
     oracle standing in for the kernel."""
 
@@ -85,6 +86,7 @@ class HostSlabRunner:
         self.n_loc = n1 - n0
         gs = n_total if group_size is None else group_size
         self.gs_loc = self.n_loc if gs >= n_total else gs
+        self.whole = (m, n_total, min(gs, n_total))
         self.b = reconn_sz
         self.r_rows = max(1, self.n_loc // self.gs_loc) * reconn_sz
         self.device = torch.device(device if device is not None else "cuda")
@@ -126,13 +128,14 @@ class HostSlabRunner:
 
     def _product_chunk(self, j):
         torch = self.torch
-        fn = self.compute or ops.oft_tn
-        kwargs = dict(group_size=self.gs_loc, reconn_sz=self.b)
-        if self.compute is None:
-            kwargs["lib"] = self.lib
         stream = torch.cuda.current_stream(self.device).cuda_stream if self.cuda else None
         rows = self.world * self.pc
-        fn(rows, self.n_loc, self.k, self.dX[j], self.k, self.dW, self.k, self.dR, self.k, self.dY[j], self.n_loc, stream, **kwargs)
+        if self.compute is None:
+            ops.oft_tn_part(self.whole, rows, self.n_loc, self.k, self.dX[j], self.k, self.dW, self.k, self.dR, self.k, [self.dY[j]], self.n_loc, stream,
+                            group_size=self.gs_loc, reconn_sz=self.b, lib=self.lib)
+        else:
+            self.compute(rows, self.n_loc, self.k, self.dX[j], self.k, self.dW, self.k, self.dR, self.k, self.dY[j], self.n_loc, stream,
+                         group_size=self.gs_loc, reconn_sz=self.b)
 
     def _download_chunk(self, hY_slab, j):
         for r in range(self.world):
@@ -238,7 +241,7 @@ class SlabProductAllGather:
         self.mode = mode
         self.world = world if world is not None else dist.get_world_size()
         self.rank = rank if rank is not None else dist.get_rank()
-        self.m, self.k, self.n_loc, self.b, self.lib = m, k, n1 - n0, reconn_sz, lib
+        self.m, self.n_total, self.k, self.n_loc, self.b, self.lib = m, n_total, k, n1 - n0, reconn_sz, lib
         self.device = torch.device(device if device is not None else f"cuda:{torch.cuda.current_device()}")
         if (n1 - n0) * self.world != n_total:
             raise ValueError("SlabProductAllGather needs equal slabs on every rank")
@@ -259,12 +262,13 @@ class SlabProductAllGather:
         torch, dist = self.torch, self.dist
         main = torch.cuda.current_stream(self.device)
         mine = self.y_all[self.rank]
+        whole = (self.m, self.n_total, self.n_total)  # slab and chunks have the bits of one oft_tn over all rows and columns
         if self.mode == "stores":
             # One launch: the kernel's epilogue stores every tile into this rank's place of every GPU's buffer (plain
-            # global stores over NVLink into the peers' symmetric memory; ops.oft_tn_gather).
+            # global stores over NVLink into the peers' symmetric memory).
             dsts = [mine] + [self.peer_views[(self.rank + p) % self.world][self.rank] for p in range(1, self.world)]
-            ops.oft_tn_gather(self.m, self.n_loc, self.k, dX, self.k, dW_slab, self.k, dR, self.k, dsts, self.n_loc, main.cuda_stream,
-                              group_size=self.n_loc, reconn_sz=self.b, lib=self.lib)
+            ops.oft_tn_part(whole, self.m, self.n_loc, self.k, dX, self.k, dW_slab, self.k, dR, self.k, dsts, self.n_loc, main.cuda_stream,
+                            group_size=self.n_loc, reconn_sz=self.b, lib=self.lib)
             main.synchronize()
             if self.world > 1:
                 dist.barrier()  # every peer's stores into this rank's buffer are complete
@@ -274,8 +278,8 @@ class SlabProductAllGather:
         i = 0
         for c0 in range(0, self.m, self.chunk_rows):
             rows = min(self.chunk_rows, self.m - c0)
-            ops.oft_tn(rows, self.n_loc, self.k, dX[c0:], self.k, dW_slab, self.k, dR, self.k, mine[c0:], self.n_loc, main.cuda_stream,
-                       group_size=self.n_loc, reconn_sz=self.b, lib=self.lib)
+            ops.oft_tn_part(whole, rows, self.n_loc, self.k, dX[c0:], self.k, dW_slab, self.k, dR, self.k, [mine[c0:]], self.n_loc, main.cuda_stream,
+                            group_size=self.n_loc, reconn_sz=self.b, lib=self.lib)
             done = torch.cuda.Event()
             done.record(main)
             for p in range(1, self.world):  # start with the next rank so that the ranks do not all write to one peer at once

@@ -76,6 +76,9 @@ def test_new_entry_points_validate_before_any_cuda_call(lib):
     assert lib.b200_oft_tn_f16_sharded(8, 16, 16, 16, 16, 0, devs, ptrs, 16, ptrs, 16, ptrs, 16, ptrs, 16, None) == ops.EINVAL  # world = 0
     assert lib.b200_oft_tn_f16_sharded(8, 16, 16, 5, 16, 1, devs, ptrs, 16, ptrs, 16, ptrs, 16, ptrs, 16, None) == ops.EINVAL  # n % group_size
     assert lib.b200_oft_tn_f16_sharded(8, 16, 16, 16, 16, 1, devs, None, 16, ptrs, 16, ptrs, 16, ptrs, 16, None) == ops.EINVAL
+    part = lambda wm, wn, wg, n, g: lib.b200_oft_tn_f16_part(wm, wn, wg, 8, n, 16, g, 16, p, 16, p, 16, p, 16, 1, ptrs, n, None)
+    assert part(8, 0, 16, 16, 16) == ops.EINVAL and part(8, 40, 16, 16, 16) == ops.EINVAL and part(8, 16, 16, 32, 32) == ops.EINVAL  # the whole's sizes
+    assert part(8, 64, 16, 32, 32) == ops.EINVAL and b"whole" in lib.b200_last_error()  # two groups of the whole as one
     with pytest.raises(ops.Error):
         ops.set_option("no_such_option", 1, lib)
     for name in ("oft_route", "raster", "tile_sync", "l2_hints", "gemm_tile_sync", "gemm_l2_hints", "gemm_split", "maps_3d", "ring_bands", "prefetch", "rot_pairs"):
