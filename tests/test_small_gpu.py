@@ -237,3 +237,41 @@ def test_rows_of_x_longer_than_a_megabyte(lib, cuda, pair_build):
         return C.view(torch.int16)
 
     assert torch.equal(run(small_tiles=0), run(oft_route=1))
+
+
+@pytest.mark.parametrize("layout", ["TN", "NT"])
+@pytest.mark.parametrize("in_type,out_type,alpha,beta", [(0, 0, 0.5, 0.0), (0, 1, 1.0 / 128, 0.0), (2, 1, -4.0, 0.0), (2, 1, 1.0, -0.25), (0, 1, 0.5, 1.0)])
+def test_scaled_products_have_the_sums_of_the_bare_one(lib, cuda, pair_build, layout, in_type, out_type, alpha, beta):
+    """What the header says of products scaled by alpha or beta, on a shape whose K is cut into pieces: the fp32 sums are
+    those of the bare product, scaled once (alpha is a power of two, so that step is exact), and the option gemm_split = 0
+    keeps K whole, with the bits of the pair kernel."""
+    if not pair_build:
+        pytest.skip("the single-CTA build never cuts K")
+    import torch
+
+    m, n, k = 264, 136, 2048
+    g = torch.Generator(device=cuda).manual_seed(97)
+    tin = torch.float16 if in_type == 0 else torch.float32
+    sa, sb = ((m, k), (n, k)) if layout == "TN" else ((k, m), (k, n))
+    A, B = (torch.randn(s, generator=g, device=cuda).to(tin) for s in (sa, sb))
+    c0 = torch.randn((n, m), generator=g, device=cuda)
+
+    def run(a, be, out=out_type, **opts):
+        import contextlib
+        C = c0.to(torch.float16 if out == 0 else torch.float32, copy=True)
+        with contextlib.ExitStack() as es:
+            for name, v in opts.items():
+                es.enter_context(ops.option(name, v, lib))
+            ops.gemm_ex(*layout, m, n, k, a, A, sa[1], B, sb[1], be, C, m, in_type=in_type, out_type=out, lib=lib)
+        assert ops.device_status(lib)[0] == 0
+        return C
+
+    sums = run(1.0, 0.0, out=1)
+    assert not torch.equal(sums, run(1.0, 0.0, out=1, gemm_split=0))  # K is cut
+    got = run(alpha, beta)
+    if beta == 0.0:
+        assert torch.equal(got, (alpha * sums).to(got.dtype))
+    else:  # one or two roundings of fp32
+        want, terms = alpha * sums.double() + beta * c0.double(), (alpha * sums.double()).abs() + (beta * c0.double()).abs()
+        assert bool(((got.double() - want).abs() <= 2.0 ** -23 * terms).all())
+    assert torch.equal(run(alpha, beta, gemm_split=0), run(alpha, beta, small_tiles=0, gemm_split=0))
