@@ -999,7 +999,8 @@ int choose_route(int m, int n, int group_size, int k, int b, bool aligned, const
   // 576 b 64 74.6 / 49.2 / 287, 2988 x 4253 x 4176 b 8 125 / 99 / 215, 39866 x 647 x 3456 b 128 254 / 260 / 298.  Short K, a wide
   // group and more tiles than SM pairs: 16589 x 4904 x 384 b 128 114 / 82 / 140 (route 4 140), 6503 x 7008 x 512 b 64 68 / 56 / 86; with one
   // round of tiles there is nothing to serialise the rotation with (647 x 4096 x 512 b 64 14.8 / 21.2 / 21.8).
-  if (g_more.n == 0 && two_pass_fits(k)) {
+  const bool group_ok = group_size == n || group_size % static_cast<int>(CurrCompParams::bN) == 0;  // what the fused routes take of these widths
+  if (g_more.n == 0 && group_ok && two_pass_fits(k)) {
     if (!aligned && group_size == n) return 2;
     const long long t256 = ((static_cast<long long>(m) + 255) / 256) * ((static_cast<long long>(group_size) + 255) / 256);
     if (wide && k_steps < 16 && t256 > st->sm_count / 2) return 2;

@@ -275,3 +275,18 @@ def test_scaled_products_have_the_sums_of_the_bare_one(lib, cuda, pair_build, la
         want, terms = alpha * sums.double() + beta * c0.double(), (alpha * sums.double()).abs() + (beta * c0.double()).abs()
         assert bool(((got.double() - want).abs() <= 2.0 ** -23 * terms).all())
     assert torch.equal(run(alpha, beta, gemm_split=0), run(alpha, beta, small_tiles=0, gemm_split=0))
+
+
+@pytest.mark.parametrize("k", [512, 2048])
+def test_wide_groups_that_no_kernel_takes_stay_refused(lib, cuda, pair_build, k):
+    """A group that is neither all of N nor a multiple or divisor of the N tile is refused whatever K is."""
+    if not pair_build:
+        pytest.skip("the single-CTA build has one route")
+    import torch
+
+    m, gs, b = 4000, 2056, 64
+    n = 2 * gs
+    X, W, R, C = (torch.zeros(s, dtype=torch.float16, device=cuda) for s in ((m, k), (n, k), (2 * b, k), (m, n)))
+    with pytest.raises(ops.Error) as e:
+        ops.oft_tn(m, n, k, X, k, W, k, R, k, C, n, group_size=gs, reconn_sz=b, lib=lib)
+    assert e.value.code == ops.EUNSUPPORTED and "group_size" in e.value.message
