@@ -254,6 +254,13 @@ def _interleaved(timed, fns, reps, rounds=4, warm=3):
     return [statistics.median(x) for x in samples]
 
 
+def compared_routes(chosen):
+    """(code, name) of the routes to time beside the chosen one; the kernel for small problems only where it is the choice."""
+    from cute_mma_b200 import ops
+
+    return [(code, name) for code, name in ops.ROUTES.items() if name != "fused_small" or name == chosen]
+
+
 def projection_shape_rates(lib, dev, stream, peaks):
     """Device-timed rates of the single-GPU projection shape (M 16384, K = N 4096, b 64, Cayley blocks) on every
     route of the library, beside the plain GEMM of the same size and cuBLAS on it: medians of 5 interleaved timings of
@@ -271,10 +278,10 @@ def projection_shape_rates(lib, dev, stream, peaks):
     dY = torch.empty((m, n), dtype=torch.float16, device=dev)
     timed = _device_timer(stream)
     fl = flops_of(m, k, n, b)
-    chosen = ops.oft_plan(m, n, k, reconn_sz=b, lib=lib)["path"]
+    chosen = ops.oft_route(m, n, k, reconn_sz=b, lib=lib)
     # every route, the plain GEMM of the same size (W . X^T, no rotation: the ceiling of any route) and cuBLAS on it, all
     # timed in turn (5 rounds of 10 launches each, medians), so that clock drift hits them alike
-    order = sorted(ops.ROUTES.items(), key=lambda kv: kv[1] != chosen)
+    order = sorted(compared_routes(chosen), key=lambda kv: kv[1] != chosen)
 
     def on_route(code):
         def call():
@@ -413,7 +420,8 @@ def run_gpu_arm(args, workload):
         return max_over_ranks(t0.elapsed_time(t1) / steps)
 
     warm = max(args.warmup, 3)
-    plan = ops.oft_plan(m, n_loc, k, reconn_sz=b, lib=lib)
+    launches = ops.oft_plan(m, n_loc, k, reconn_sz=b, lib=lib)["kernel_launches"]
+    chosen = ops.oft_route(m, n_loc, k, reconn_sz=b, lib=lib)
     for _ in range(warm):
         step()
     barrier()
@@ -431,9 +439,9 @@ def run_gpu_arm(args, workload):
 
     # every route of the library on the same workload, same steps, max over ranks
     peaks = measured_peaks()
-    routes = {plan["path"]: {"ms_per_step": ms, "value": value, "unit": "TFLOP/s", "steps": args.steps, "chosen": True}}
-    for code, rname in ops.ROUTES.items():
-        if rname == plan["path"]:
+    routes = {chosen: {"ms_per_step": ms, "value": value, "unit": "TFLOP/s", "steps": args.steps, "chosen": True}}
+    for code, rname in compared_routes(chosen):
+        if rname == chosen:
             continue
         with ops.option("oft_route", code, lib):
             r_ms = timed_steps(args.steps, 2)
@@ -443,7 +451,7 @@ def run_gpu_arm(args, workload):
             routes[rname]["same_bits_as_chosen"] = bool(torch.equal(y_chosen.view(torch.int16), dY.view(torch.int16)))
     del y_chosen
     # the chosen route once more, after the others: the first timing ran on the coolest GPU of this process
-    routes[plan["path"]]["ms_per_step_after_the_others"] = timed_steps(args.steps, 2)
+    routes[chosen]["ms_per_step_after_the_others"] = timed_steps(args.steps, 2)
     for r in routes.values():
         r["frac_of_measured_bf16_burst_per_gpu"] = r["value"] / world / peaks["bf16_burst"]
     # the two passes of the two-pass route on their own (rank 0's GPU)
@@ -540,13 +548,14 @@ def run_gpu_arm(args, workload):
         achieved = flops_launch / (ms * 1e-3) * 1e-12
         timed_s = ms * args.steps * 1e-3
         peak = peaks["bf16_sustained"] if timed_s >= 2.0 else peaks["bf16_burst"]
-        kernel_of = {"fused_ring": "oft3_kernel", "fused_ring_split": "oft4_kernel", "fused_tmem": "oft2_kernel", "two_pass": "xr_kernel + gemm2_kernel"}
+        kernel_of = {"fused_ring": "oft3_kernel", "fused_ring_split": "oft4_kernel", "fused_tmem": "oft2_kernel", "two_pass": "xr_kernel + gemm2_kernel",
+                     "fused_small": "small_kernel"}
         config_of_route = {"fused_ring": "oft_ring", "fused_ring_split": "oft_ring_split"}
         roofline = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                     "peak_source": f"{peaks['source']} bf16 {'sustained' if timed_s >= 2.0 else 'burst'} (cuBLAS matmul on this pool)",
-                    "traffic": (NCU_TRAFFIC_BYTES.get((workload, plan["path"])) if world == 1 else None),
-                    "frac_of_nominal_fp16": achieved / NOMINAL_FP16_TFLOPS, "route": plan["path"], "kernel": kernel_of[plan["path"]],
-                    "launch_ms": ms, "kernel_config": ops.kernel_info(lib)[config_of_route.get(plan["path"], "oft")], "n_per_gpu": n_loc,
+                    "traffic": (NCU_TRAFFIC_BYTES.get((workload, chosen)) if world == 1 else None),
+                    "frac_of_nominal_fp16": achieved / NOMINAL_FP16_TFLOPS, "route": chosen, "kernel": kernel_of[chosen],
+                    "launch_ms": ms, "kernel_config": ops.kernel_info(lib)[config_of_route.get(chosen, "oft")], "n_per_gpu": n_loc,
                     "routes": routes}
         line = {
             "metric": METRIC, "value": value, "unit": "TFLOP/s", "n_gpus": world, "steps": args.steps, "warmup": warm,
@@ -555,7 +564,7 @@ def run_gpu_arm(args, workload):
             "e2e": {"value": total_flops / e2e_s * 1e-12, "unit": "TFLOP/s", "h2d_bytes_per_step": int(th[0].item()),
                     "d2h_bytes_per_step": int(th[1].item()), "ms_per_step": e2e_s * 1e3, "steps": args.e2e_steps,
                     "api": e2e_api, "matches_device_path": same},
-            "gpu_launches": args.steps * world * plan["kernel_launches"], "clocks": clocks,
+            "gpu_launches": args.steps * world * launches, "clocks": clocks,
         }
         if e2e_legs is not None:
             line["e2e"]["legs_ms"] = e2e_legs

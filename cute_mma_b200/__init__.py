@@ -16,9 +16,11 @@ from .ops import (  # noqa: F401
     kernel_info,
     lora_tn,
     oft_plan,
+    oft_route,
     oft_tn,
     oft_tn_a_rw,
     oft_tn_host,
+    oft_tn_part,
     oft_tn_static,
     oft_tn_two_pass,
     rotate,

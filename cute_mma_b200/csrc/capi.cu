@@ -1385,7 +1385,7 @@ int b200_oft_plan(int m, int n, int k, int group_size, int reconn_sz, int* path,
   int pieces = 1;
   const int route = choose_route(m, n, group_size, k, reconn_sz == 8 ? 16 : reconn_sz, n % 8 == 0, st, &pieces);  // C packed and aligned
   // small_kernel forms X.R per tile of C on the chip and needs no scratch, like the kernel of route 1; a caller of the
-  // plan sees the same 1 for both unless it asked for 5 itself
+  // plan sees the same 1 for both unless it asked for 5 itself (b200_oft_route tells them apart)
   if (path) *path = route == 5 && opt(kOptOftRoute) != 5 ? 1 : route;
   const int groups = n / group_size;
   int launches = route == 3 || route == 4 ? groups : 1;
@@ -1394,6 +1394,17 @@ int b200_oft_plan(int m, int n, int k, int group_size, int reconn_sz, int* path,
     launches = 2 * groups * static_cast<int>((m + rows - 1) / rows);
   }
   if (kernel_launches) *kernel_launches = launches + (reconn_sz == 8 ? 1 : 0);
+  return B200_OK;
+}
+
+int b200_oft_route(int m, int n, int k, int group_size, int reconn_sz, int c_aligned, int* route) {
+  g_err.clear();
+  if (m <= 0 || n <= 0 || k <= 0 || group_size <= 0 || reconn_sz <= 0 || n % group_size != 0 || k % reconn_sz != 0 || !route)
+    return fail(B200_EINVAL, "bad route arguments (m=%d n=%d k=%d group_size=%d reconn_sz=%d)", m, n, k, group_size, reconn_sz);
+  DeviceState* st;
+  if (int rc = device_state(&st)) return rc;
+  int pieces = 1;
+  *route = choose_route(m, n, group_size, k, reconn_sz == 8 ? 16 : reconn_sz, c_aligned != 0, st, &pieces);
   return B200_OK;
 }
 

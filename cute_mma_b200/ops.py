@@ -25,7 +25,7 @@ OK, EINVAL, EUNSUPPORTED, ECUDA, EDEVICE = 0, 1, 2, 3, 4
 SYMBOLS = (
     "b200_oft_tn_f16", "b200_oft_tn_f16_two_pass", "b200_rotate_f16", "b200_oft_plan", "b200_oft_tn_f16_host", "b200_oft_tn_f16_static", "b200_transform_weight_f16", "b200_oft_tn_f16_a_rw", "b200_gemm_tn_f16", "b200_gemm_nt_f16", "b200_gemm_tn_tf32",
     "b200_gemm_nt_tf32", "b200_gemm", "b200_gemm_tn_f16_acc2", "b200_lora_tn_f16", "b200_gemm_rowmajor", "b200_peer_copy_async", "b200_shard_range", "b200_tile_coord", "b200_device_status", "b200_selftest_wait_timeout", "b200_wait_profile", "b200_kernel_info",
-    "b200_last_error", "b200_shutdown", "b200_static_status", "b200_set_option", "b200_get_option", "b200_gemm_ex", "b200_oft_tn_f16_sharded", "b200_oft_tn_f16_gather", "b200_oft_tn_f16_part",
+    "b200_last_error", "b200_shutdown", "b200_static_status", "b200_set_option", "b200_get_option", "b200_gemm_ex", "b200_oft_tn_f16_sharded", "b200_oft_tn_f16_gather", "b200_oft_tn_f16_part", "b200_oft_route",
 )
 
 
@@ -58,6 +58,7 @@ def load_library(path: str | None = None):
     lib.b200_oft_tn_f16_two_pass.argtypes = [i, i, i, i, i, vp, i, vp, i, vp, i, vp, i, vp]
     lib.b200_rotate_f16.argtypes = [i, i, i, vp, i, vp, i, vp, i, vp]
     lib.b200_oft_plan.argtypes = [i, i, i, i, i, ctypes.POINTER(i), ctypes.POINTER(i)]
+    lib.b200_oft_route.argtypes = [i, i, i, i, i, i, ctypes.POINTER(i)]
     lib.b200_oft_tn_f16_a_rw.argtypes = [i, i, i, i, i, vp, i, vp, i, vp, i, vp, i, vp]
     lib.b200_transform_weight_f16.argtypes = [i, i, i, i, vp, i, vp, i, vp, i, vp]
     lib.b200_oft_tn_f16_host.argtypes = [i, i, i, i, i, vp, i, vp, i, vp, i, vp, i]
@@ -144,11 +145,22 @@ def oft_plan(m, n, k, *, group_size=None, reconn_sz=8, lib=None) -> dict:
     library's kernels per oft_tn call}: fused_tmem keeps X.R in tensor memory per N tile, fused_ring shares one X.R
     per row block among the N tiles of a group through an L2-resident ring (fused_ring_split: with the rotation on
     SM pairs of its own), two_pass writes X.R to memory first.  Small problems run on a kernel of their own that forms
-    X.R per tile too and are reported as fused_tmem ('fused_small' when the option "oft_route" is 5)."""
+    X.R per tile too and are reported as fused_tmem ('fused_small' when the option "oft_route" is 5); oft_route tells the
+    two apart."""
     lib = lib or load_library()
     path, launches = ctypes.c_int(0), ctypes.c_int(0)
     _check(lib, lib.b200_oft_plan(m, n, k, n if group_size is None else group_size, reconn_sz, ctypes.byref(path), ctypes.byref(launches)))
     return {"path": ROUTES[path.value], "kernel_launches": launches.value}
+
+
+def oft_route(m, n, k, *, group_size=None, reconn_sz=8, c_aligned=None, lib=None) -> str:
+    """Name of the route oft_tn takes: 'fused_small' for small problems, else oft_plan's 'path'.  ``c_aligned`` (rows of
+    C on 16-byte boundaries) defaults to a packed C."""
+    lib = lib or load_library()
+    route = ctypes.c_int(0)
+    aligned = n % 8 == 0 if c_aligned is None else c_aligned
+    _check(lib, lib.b200_oft_route(m, n, k, n if group_size is None else group_size, reconn_sz, int(aligned), ctypes.byref(route)))
+    return ROUTES[route.value]
 
 
 def set_option(name: str, value: int, lib=None) -> None:

@@ -290,3 +290,23 @@ def test_wide_groups_that_no_kernel_takes_stay_refused(lib, cuda, pair_build, k)
     with pytest.raises(ops.Error) as e:
         ops.oft_tn(m, n, k, X, k, W, k, R, k, C, n, group_size=gs, reconn_sz=b, lib=lib)
     assert e.value.code == ops.EUNSUPPORTED and "group_size" in e.value.message
+
+
+def test_route_names_the_kernel_that_runs(lib, cuda, pair_build):
+    """oft_plan reports small problems as fused_tmem (X.R formed per tile, no scratch), oft_route by their own name; both
+    agree elsewhere, and rows of C off 16-byte boundaries count."""
+    if not pair_build:
+        pytest.skip("the single-CTA build has one route")
+    assert ops.oft_plan(8, 4096, 4096, reconn_sz=64, lib=lib) == {"path": "fused_tmem", "kernel_launches": 1}
+    assert ops.oft_route(8, 4096, 4096, reconn_sz=64, lib=lib) == "fused_small"
+    with ops.option("small_tiles", 0, lib):
+        assert ops.oft_route(8, 1024, 4096, reconn_sz=64, lib=lib) == "fused_tmem"
+    for m, n, k, b, gs in ((16384, 4096, 4096, 64, None), (8192, 8192, 8192, 8, 256), (65536, 28672, 8192, 128, None), (6503, 7008, 512, 64, None)):
+        assert ops.oft_route(m, n, k, group_size=gs, reconn_sz=b, lib=lib) == ops.oft_plan(m, n, k, group_size=gs, reconn_sz=b, lib=lib)["path"]
+    assert ops.oft_route(16384, 4096, 4096, reconn_sz=64, c_aligned=False, lib=lib) == "two_pass"
+    for route, name in ops.ROUTES.items():
+        with ops.option("oft_route", route, lib):
+            assert ops.oft_route(384, 2048, 512, reconn_sz=64, lib=lib) == name
+    with pytest.raises(ops.Error) as e:
+        ops.oft_route(8, 4096, 4100, reconn_sz=64, lib=lib)
+    assert e.value.code == ops.EINVAL
