@@ -397,6 +397,17 @@ int small_pieces(const SmallKind& kind, int m, int n, int k, const DeviceState* 
   return split < p.steps / kind.unit ? split : p.steps / kind.unit;
 }
 
+// Further destinations of the result, set by b200_oft_tn_f16_gather for its own call: the shared-X.R kernel and the
+// kernel for small problems store every tile to each of them from their epilogues (plain stores; the buffers may be
+// another GPU's memory mapped into this process).  `stored` tells the entry point whether a launch took them; otherwise
+// it copies.
+struct MoreDst {
+  int n = 0;
+  __half* p[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+  bool stored = false;
+};
+thread_local MoreDst g_more;
+
 template <class T>
 int launch_small(int split, int m, int n, int k, const void* P, int ldP, const char* p_name, const void* Q, int ldQ, const char* q_name,
                  const void* R, int ldR, int group_size, void* C, int ldC, float alpha, float beta, cudaStream_t stream, DeviceState* st) {
@@ -422,24 +433,40 @@ int launch_small(int split, int m, int n, int k, const void* P, int ldP, const c
   }
   const int vec = (reinterpret_cast<uintptr_t>(C) % (4 * sizeof(TOut))) == 0 && ldC % 4 == 0;
   const int tiles_m = (m + 127) / 128, tiles_n = (n + 127) / 128;
-  SmallArgs args{m, n, k, C, ldC, st->status, p.n_tile, tiles_n, split, p.stages, p.xbufs, group_size, p3d, q3d, vec, alpha, beta};
-  auto kernel = small_kernel<T>;
-  if (int rc = opt_in_smem(kernel, kWholeSmBytes)) return rc;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(static_cast<unsigned>(tiles_m * tiles_n * split));
-  cfg.blockDim = dim3(T::kThreads);
-  cfg.dynamicSmemBytes = static_cast<size_t>(p.smem);
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = opt(kOptPdl) != 0 ? 1 : 0;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = static_cast<unsigned>(split);
-  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = split > 1 ? 2 : 1;
-  CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, mp, mq, mr, args));
-  return B200_OK;
+  const SmallArgs args{m, n, k, C, ldC, st->status, p.n_tile, tiles_n, split, p.stages, p.xbufs, group_size, p3d, q3d, vec, alpha, beta};
+  auto launch = [&](auto kernel, const auto& kernel_args) -> int {
+    if (int rc = opt_in_smem(kernel, kWholeSmBytes)) return rc;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(tiles_m * tiles_n * split));
+    cfg.blockDim = dim3(T::kThreads);
+    cfg.dynamicSmemBytes = static_cast<size_t>(p.smem);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = opt(kOptPdl) != 0 ? 1 : 0;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = static_cast<unsigned>(split);
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = split > 1 ? 2 : 1;
+    CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, mp, mq, mr, kernel_args));
+    return B200_OK;
+  };
+  if constexpr (T::kRot) {
+    if (g_more.n > 0) {
+      SmallArgsMore more;
+      static_cast<SmallArgs&>(more) = args;
+      more.n_more = g_more.n;
+      for (int d = 0; d < g_more.n; ++d) {
+        more.C_more[d] = g_more.p[d];
+        if (reinterpret_cast<uintptr_t>(g_more.p[d]) % (4 * sizeof(TOut)) != 0) more.vec = 0;
+      }
+      const int rc = launch(small_kernel<T, true>, more);
+      g_more.stored = rc == B200_OK;
+      return rc;
+    }
+  }
+  return launch(small_kernel<T>, args);
 }
 
 // (A pair kernel with half the N extent was tried for evening out the last wave of tiles and for small problems:
@@ -811,16 +838,6 @@ RingPlan ring_plan(int m, int n, int k, const DeviceState* st) {
   return p;
 }
 
-// Further destinations of the result, set by b200_oft_tn_f16_gather for its own call: the shared-X.R kernel stores
-// every tile to each of them from its epilogue (plain stores; the buffers may be another GPU's memory mapped into
-// this process).  `stored` tells the entry point whether a launch took them; otherwise it copies.
-struct MoreDst {
-  int n = 0;
-  __half* p[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-  bool stored = false;
-};
-thread_local MoreDst g_more;
-
 // Scratch of one ring launch, stream-ordered from the library's pool: zeroed counters, then the ring.
 struct RingScratch {
   unsigned char* base = nullptr;
@@ -1006,7 +1023,7 @@ int choose_route(int m, int n, int group_size, int k, int b, bool aligned, const
     if (wide && k_steps < 16 && t256 > st->sm_count / 2) return 2;
   }
   if (!wide) return 1;
-  if (g_more.n > 0) return 3;  // only oft3_kernel stores to further destinations
+  if (g_more.n > 0) return 3;  // of the ring kernels, only oft3_kernel stores to further destinations
   // Route 4 also wants long tiles: its product pairs write C with the plain GEMM's epilogue (one 2-byte store per
   // element), which must fit beside a tile's MMAs.  Interleaved runs, route 4 / route 3 time: M 32768, N 28672, K 1024,
   // b 64: 1.61; M 262144, N 12288, K 2048, b 64 (3 pairs): 1.05; M 65536, N 28672, b 128 (2 pairs), K 2048: 0.86,
@@ -1263,7 +1280,7 @@ int oft_gather(int m, int n, int k, int group_size, int b, const void* A, int ld
   const bool stored = g_more.stored;
   g_more = MoreDst{};
   if (rc != B200_OK || stored || m == 0 || n == 0) return rc;
-  // a route without the multi-destination epilogue (few N tiles per group, k = 0, no scratch): copy the result
+  // a route without the multi-destination epilogue (few N tiles per group of a larger problem, k = 0, no scratch): copy the result
   for (int d = 1; d < n_dst; ++d)
     CUDA_TRY(cudaMemcpy2DAsync(C_dst[d], static_cast<size_t>(ldC) * 2, C_dst[0], static_cast<size_t>(ldC) * 2, static_cast<size_t>(n) * 2, m,
                                cudaMemcpyDeviceToDevice, stream));

@@ -79,3 +79,28 @@ def make_oft_case(m, n, k, b, group_size=None, seed=0, kind="qr", xdist="uniform
     else:
         blocks = inputs.blocks_structured(G, k // b, b)
     return A, inputs.pack_r(blocks), B
+
+
+def graph_node_types(fn):
+    """Types of the nodes (cudaGraphNodeType values) of the CUDA graph that ``fn()`` is captured into; nothing runs.
+    ``fn`` launches on torch's current stream and has run once before."""
+    import ctypes
+
+    import torch
+
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        fn()
+    rt = ctypes.CDLL("libcudart.so.12")
+    raw, count = ctypes.c_void_p(graph.raw_cuda_graph()), ctypes.c_size_t(0)
+    assert rt.cudaGraphGetNodes(raw, None, ctypes.byref(count)) == 0
+    nodes, types = (ctypes.c_void_p * count.value)(), []
+    assert rt.cudaGraphGetNodes(raw, nodes, ctypes.byref(count)) == 0
+    for node in nodes:
+        kind = ctypes.c_int(-1)
+        assert rt.cudaGraphNodeGetType(ctypes.c_void_p(node), ctypes.byref(kind)) == 0
+        types.append(kind.value)
+    return types
+
+
+GRAPH_KERNEL, GRAPH_MEMCPY, GRAPH_MEM_ALLOC = 0, 1, 10

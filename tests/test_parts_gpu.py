@@ -1,11 +1,11 @@
-"""Parts of one product (row chunks, slabs of N) have the bits of a single call on the whole of it,
+"""Parts of one product (row chunks, slabs of N, several destinations) have the bits of a single call on the whole of it,
 also where the library cuts K into pieces: it then does so by the whole product's sizes."""
 import types
 
 import numpy as np
 import pytest
 
-from _util import make_oft_case
+from _util import GRAPH_KERNEL, GRAPH_MEMCPY, graph_node_types, make_oft_case
 from cute_mma_b200 import ops, sharded
 
 pytestmark = pytest.mark.gpu
@@ -99,3 +99,34 @@ def test_slab_with_overlapped_all_gather_has_the_bits_of_the_whole(lib, cuda, pa
     assert ops.device_status(lib)[0] == 0
     for buf in (mine, peer):
         assert torch.equal(buf[1].view(torch.int16), want[:, n // 2:]) and not bool(buf[0].any())
+
+
+# wide group of few rows, K cut / whole; narrow; odd ldC and an 8-byte base that not every destination has
+@pytest.mark.parametrize("m,n,k,b,gs,pad", [(16, 4096, 4096, 64, None, 0), (16, 2304, 320, 32, None, 8), (200, 640, 1024, 128, None, 8), (130, 2055, 1088, 16, None, 3),
+                                            (33, 512, 1024, 8, 256, 0)])
+def test_small_gather_is_one_launch_with_the_bits_of_the_plain_call(lib, cuda, pair_build, m, n, k, b, gs, pad):
+    """Small problems store to all destinations from the kernel, as the wide groups of the shared-X.R kernel do: no copy
+    follows the launch."""
+    if not pair_build:
+        pytest.skip("the single-CTA build copies")
+    import torch
+
+    _, (dA, dR, dB) = _operands(cuda, m, n, k, b, gs, 104)
+    want = _whole(lib, cuda, dA, dR, dB, m, n, k, b, gs)
+    ldc = n + pad
+    for shift in (0, 2):  # elements by which the second destination's base is off a 16-byte boundary
+        bufs = [torch.full(((m + 1) * ldc + 2,), -7.0, dtype=torch.float16, device=cuda) for _ in range(3)]
+        dsts = [x.data_ptr() + (2 * shift if i == 1 else 0) for i, x in enumerate(bufs)]
+
+        def call():
+            ops.oft_tn_gather(m, n, k, dA, k, dB, k, dR, k, dsts, ldc, torch.cuda.current_stream(), group_size=gs, reconn_sz=b, lib=lib)
+
+        call()
+        assert ops.device_status(lib)[0] == 0
+        for i, x in enumerate(bufs):
+            off = shift if i == 1 else 0
+            rows = x[off: off + (m + 1) * ldc].view(m + 1, ldc)
+            assert torch.equal(rows[:m, :n].contiguous().view(torch.int16), want), (shift, i)
+            assert bool((rows[m] == -7.0).all()) and bool((rows[:m, n:] == -7.0).all()) and bool((x[:off] == -7.0).all())
+        kinds = graph_node_types(call)
+        assert GRAPH_MEMCPY not in kinds and kinds.count(GRAPH_KERNEL) == (2 if b == 8 else 1)  # 8 x 8 blocks: R is expanded first
