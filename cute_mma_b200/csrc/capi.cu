@@ -1000,6 +1000,9 @@ bool oft_takes_small(const Whole& w, int m, int n, int group_size, int k, int b,
   return small_group_ok(n, group_size, b) && small_oft_wins(m, n, k, b, 1, aligned, st);
 }
 
+// Groups wide enough for the kernels that share one X.R per row block among N tiles.
+bool wide_group(int group_size, int b) { return group_size >= (b >= 128 ? 4 : 8) * static_cast<int>(CurrCompParams::bN); }
+
 // aligned: rows of C start on 16-byte boundaries.  *pieces: those of K on route 5.
 int choose_route(int m, int n, int group_size, int k, int b, bool aligned, const DeviceState* st, int* pieces) {
   int path = g_oft_path != 0 ? g_oft_path : opt(kOptOftRoute);
@@ -1009,8 +1012,8 @@ int choose_route(int m, int n, int group_size, int k, int b, bool aligned, const
   if (path == 2 || path == 3 || path == 4 || path == 5) return can_share ? path : 1;
   if (path == 1 || !can_share) return 1;
   if (opt(kOptSmallTiles) != 0 && oft_takes_small(w, m, n, group_size, k, b, aligned, st, pieces)) return 5;
-  const int k_steps = (k + 63) / 64, min_tiles = b >= 128 ? 4 : 8;
-  const bool wide = group_size >= min_tiles * static_cast<int>(CurrCompParams::bN);
+  const int k_steps = (k + 63) / 64;
+  const bool wide = wide_group(group_size, b);
   // Rotation pass + plain GEMM (route 2).  Rows of C that are not 16-byte aligned and one group: the fused kernels store
   // them a row at a time after a transpose in registers (route 1) or element by element (route 3); us on routes 1 / 2 / 3: 12375 x 1473 x
   // 576 b 64 74.6 / 49.2 / 287, 2988 x 4253 x 4176 b 8 125 / 99 / 215, 39866 x 647 x 3456 b 128 254 / 260 / 298.  Short K, a wide
@@ -1033,6 +1036,12 @@ int choose_route(int m, int n, int group_size, int k, int b, bool aligned, const
   return split ? 4 : 3;
 }
 
+bool is_capturing(cudaStream_t stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) cudaGetLastError();
+  return status == cudaStreamCaptureStatusActive;
+}
+
 // group_size == n or a multiple of the N tile: one R per tile.  group_size a divisor of the N tile (the
 // reference's bN % group_size == 0 case, cute_oft_coop_pc.cu:383): bN / group_size groups per tile, pair kernel.
 template <int kB>
@@ -1041,8 +1050,10 @@ int launch_oft(int m, int n, int k, int group_size, const void* A, int ldA, cons
   constexpr int kBN = CurrCompParams::bN;
   int pieces = 1;
   const int route = choose_route(m, n, group_size, k, kB, (reinterpret_cast<uintptr_t>(C) & 15) == 0 && (ldC & 7) == 0, st, &pieces);
-  if (route == 2) {
-    const bool own = g_oft_path != 2 && opt(kOptOftRoute) != 2;
+  const bool own = g_oft_path != 2 && opt(kOptOftRoute) != 2;
+  // A captured call allocates nodes of its graph, which then can be no child graph or conditional body: narrow groups,
+  // which no other route needs scratch for, stay off the two passes there.
+  if (route == 2 && !(own && !wide_group(group_size, kB) && is_capturing(stream))) {
     const int rc = oft_two_pass<kB>(m, n, k, group_size, A, ldA, B, ldB, R, ldR, C, ldC, stream, st, own);
     if (rc != kNoScratch) return rc;
     if (g_oft_path == 2) return fail(B200_ECUDA, "no device memory for the %lld bytes of X.R scratch", static_cast<long long>(m) * ((k + 7) & ~7) * 2);

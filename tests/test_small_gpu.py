@@ -3,7 +3,7 @@ rotation buffers, against the routes it replaces (bit for bit where K is not cut
 import numpy as np
 import pytest
 
-from _util import make_oft_case, truth_ok
+from _util import GRAPH_MEM_ALLOC, graph_node_types, make_oft_case, truth_ok
 from cute_mma_b200 import ops
 from oracle import oracle
 
@@ -310,3 +310,83 @@ def test_route_names_the_kernel_that_runs(lib, cuda, pair_build):
     with pytest.raises(ops.Error) as e:
         ops.oft_route(8, 4096, 4100, reconn_sz=64, lib=lib)
     assert e.value.code == ops.EINVAL
+
+
+@pytest.mark.parametrize("m,n,k,b", [(5000, 1473, 576, 64), (4000, 647, 1152, 128)])
+def test_narrow_unaligned_products_are_captured_without_scratch(lib, cuda, pair_build, m, n, k, b):
+    """Rows of C that are not 16-byte aligned, a narrow group: the rotation pass + GEMM outside of a capture, the kernel
+    that needs no scratch inside (a graph with allocation nodes could be no child graph or conditional body); the same
+    bits."""
+    if not pair_build:
+        pytest.skip("the single-CTA build has one route")
+    import torch
+
+    g = torch.Generator(device=cuda).manual_seed(99)
+    X = torch.randn((m, k), generator=g, device=cuda).half()
+    W = (torch.randn((n, k), generator=g, device=cuda) * 0.02).half()
+    R = (torch.randn((b, k), generator=g, device=cuda) * 0.1).half()
+    C = torch.zeros((m, n), dtype=torch.float16, device=cuda)
+
+    def call():
+        ops.oft_tn(m, n, k, X, k, W, k, R, k, C, n, torch.cuda.current_stream(), reconn_sz=b, lib=lib)
+
+    call()
+    torch.cuda.synchronize()
+    want = C.clone()
+    assert GRAPH_MEM_ALLOC not in graph_node_types(call)
+    C.zero_()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert ops.device_status(lib)[0] == 0
+    assert torch.equal(C.view(torch.int16), want.view(torch.int16))
+
+
+def test_dependent_launch_behind_two_streams(lib, cuda, pair_build):
+    """A product whose operands come from two streams joined by an event, run and captured: the launch that may start
+    early waits for both producers."""
+    if not pair_build:
+        pytest.skip("the single-CTA build has no dependent launches")
+    import torch
+
+    m, n, k = 24, 1024, 1024
+    g = torch.Generator(device=cuda).manual_seed(100)
+    W0 = (torch.randn((n, k), generator=g, device=cuda) / 32).half()
+    X0 = torch.randn((m, k), generator=g, device=cuda).half()
+    big = torch.randn((4096, 4096), generator=g, device=cuda)
+    want = torch.empty((m, n), dtype=torch.float16, device=cuda)
+    ops.gemm_tn(n, m, k, W0, k, X0, k, want, n, lib=lib)
+    torch.cuda.synchronize()
+    W, X, C = torch.zeros_like(W0), torch.zeros_like(X0), torch.zeros_like(want)
+    side, scratch = torch.cuda.Stream(), torch.zeros_like(big)
+
+    def step():
+        main = torch.cuda.current_stream()
+        side.wait_stream(main)
+        with torch.cuda.stream(side):
+            for _ in range(3):
+                torch.add(big, big, out=scratch)  # keeps the side stream busy in front of the copy
+            W.copy_(W0)
+        X.copy_(X0)
+        main.wait_stream(side)
+        ops.gemm_tn(n, m, k, W, k, X, k, C, n, main, lib=lib)
+
+    def check():
+        torch.cuda.synchronize()
+        assert ops.device_status(lib)[0] == 0
+        assert torch.equal(C, want)
+        W.zero_(), X.zero_(), C.zero_()
+
+    s = torch.cuda.Stream()
+    for _ in range(3):
+        with torch.cuda.stream(s):
+            step()
+        check()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        step()
+    for _ in range(3):
+        graph.replay()
+        check()
