@@ -327,9 +327,11 @@ thread_local bool g_whole_k = false;
 // 0.72 us per step between them (both operands of a 128-wide tile are read from shared memory at its full rate), plus
 // the fixed costs and 1.5 us of epilogue per round.  1848 x 1488 x 489 half: 8.9 against 12.8 us; 2904 x 960 x 11305: 110
 // against 70 us.
-bool small_wins(int m, int n, int steps, const DeviceState* st) {
+// With K whole (the passes of oft_two_pass) up to 64 K steps only in the first range: 96 tiles of 64 steps 29.6 against 36.9
+// us on the pair kernel, 128 tiles of 226 steps 97.9 against 85.
+bool small_wins(int m, int n, int steps, bool whole_k, const DeviceState* st) {
   const long long t128 = tiles_128(m, n), pairs = st->sm_count / 2;
-  if (t128 <= st->sm_count) return true;
+  if (t128 <= st->sm_count) return !whole_k || steps <= 64;
   const long long t256 = ((static_cast<long long>(m) + 255) / 256) * ((static_cast<long long>(n) + 255) / 256);
   const double rounds = static_cast<double>(t128) / (2.0 * st->sm_count);
   const double small = 5.0 + (rounds > 1.0 ? rounds : 1.0) * (0.72 * steps + 1.5);
@@ -501,9 +503,9 @@ int launch_gemm_bn(int m, int n, int k, const void* A, int ldA, const void* B, i
   DeviceState* st;
   if (int rc = device_state(&st)) return rc;
   if constexpr (kPair) {
-    if (k2 == 0 && !g_whole_k && (opt(kOptSmallTiles) < 0 ? small_wins(m, n, (k + T1::kBK - 1) / T1::kBK, st) : opt(kOptSmallTiles) != 0)) {
+    if (k2 == 0 && (opt(kOptSmallTiles) < 0 ? small_wins(m, n, (k + T1::kBK - 1) / T1::kBK, g_whole_k, st) : opt(kOptSmallTiles) != 0)) {
       using TS = SmallTraits<TIn, TOut, kNT, 0>;
-      return launch_small<TS>(small_pieces(small_kind<TS>(), m, n, k, st), m, n, k, A, ldA, "A", B, ldB, "B", nullptr, 0, 1, C, ldC, alpha, beta, stream, st);
+      return launch_small<TS>(g_whole_k ? 1 : small_pieces(small_kind<TS>(), m, n, k, st), m, n, k, A, ldA, "A", B, ldB, "B", nullptr, 0, 1, C, ldC, alpha, beta, stream, st);
     }
   }
   constexpr int kBoxN = kPair ? T2::kBNHalf : T1::kBN;

@@ -135,7 +135,10 @@ def test_small_products_chained_on_two_streams(lib, cuda, pair_build):
     (2304, 2303, 448, 32, None, 2),       # unaligned, more than two 128 x 128 tiles per SM
     (4400, 4104, 320, 8, None, 2),        # aligned, K below 1024 and more tiles than SM pairs
     (2176, 2048, 136, 8, None, 1),        # two tiles per SM, little to do: the small-problem kernel
-    (4608, 4096, 576, 64, 2048, 2)])      # two wide groups
+    (4608, 4096, 576, 64, 2048, 2),       # two wide groups
+    (3, 65536, 448, 64, None, 2),         # few rows, a very wide group: the passes' GEMM is the small-problem kernel's
+    (1, 40001, 1536, 32, None, 2),
+    (1100, 1500, 8192, 128, None, 2)])    # a GEMM that would be cut by itself
 def test_choice_between_the_routes_is_invisible(lib, cuda, pair_build, m, n, k, b, gs, want):
     """Shapes either side of the lines between the small-problem kernel, the rotation pass + GEMM and the fused kernels:
     the library's choice has the bits of the kernel that forms X.R per N tile, with aligned and unaligned rows of C."""
