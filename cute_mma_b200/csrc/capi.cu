@@ -364,8 +364,8 @@ struct SmallPlan {
   long long slots;       // CTAs resident at once
 };
 constexpr int kWholeSmBytes = 232448;
-// Geometry for P [m][k], Q [n][k] (rotated if the kind says so), K in one piece.
-SmallPlan small_plan(const SmallKind& kind, int m, int n, int k, const DeviceState* st) {
+// Geometry for a Q of [n][k] (rotated if the kind says so); P always gives a tile 128 rows.
+SmallPlan small_plan(const SmallKind& kind, int n, int k, const DeviceState* st) {
   constexpr int half_sm = 113 * 1024;
   SmallPlan p;
   p.steps = (k + kind.bk * kind.unit - 1) / (kind.bk * kind.unit) * kind.unit;
@@ -388,8 +388,7 @@ SmallPlan small_plan(const SmallKind& kind, int m, int n, int k, const DeviceSta
 }
 // Pieces along K of an m x n product: as many as there is room for CTAs at once; at least four K steps each, and none
 // below 16 steps (a K loop of 16 steps takes about 4 us, adding up the pieces 1.5).
-int small_pieces(const SmallKind& kind, int m, int n, int k, const DeviceState* st) {
-  const SmallPlan p = small_plan(kind, m, n, k, st);
+int small_pieces(const SmallKind& kind, const SmallPlan& p, int m, int n) {
   const long long tiles = tiles_128(m, n);
   int split = 1;
   if (p.steps >= 16)
@@ -411,11 +410,10 @@ struct MoreDst {
 thread_local MoreDst g_more;
 
 template <class T>
-int launch_small(int split, int m, int n, int k, const void* P, int ldP, const char* p_name, const void* Q, int ldQ, const char* q_name,
+int launch_small(const SmallPlan& p, int split, int m, int n, int k, const void* P, int ldP, const char* p_name, const void* Q, int ldQ, const char* q_name,
                  const void* R, int ldR, int group_size, void* C, int ldC, float alpha, float beta, cudaStream_t stream, DeviceState* st) {
   using TIn = typename T::TIn;
   using TOut = typename T::TOut;
-  const SmallPlan p = small_plan(small_kind<T>(), m, n, k, st);
   CUtensorMap mp, mq, mr;
   int p3d = 0, q3d = 0;
   if constexpr (!T::kMn) {
@@ -505,7 +503,8 @@ int launch_gemm_bn(int m, int n, int k, const void* A, int ldA, const void* B, i
   if constexpr (kPair) {
     if (k2 == 0 && (opt(kOptSmallTiles) < 0 ? small_wins(m, n, (k + T1::kBK - 1) / T1::kBK, g_whole_k, st) : opt(kOptSmallTiles) != 0)) {
       using TS = SmallTraits<TIn, TOut, kNT, 0>;
-      return launch_small<TS>(g_whole_k ? 1 : small_pieces(small_kind<TS>(), m, n, k, st), m, n, k, A, ldA, "A", B, ldB, "B", nullptr, 0, 1, C, ldC, alpha, beta, stream, st);
+      const SmallPlan p = small_plan(small_kind<TS>(), n, k, st);
+      return launch_small<TS>(p, g_whole_k ? 1 : small_pieces(small_kind<TS>(), p, m, n), m, n, k, A, ldA, "A", B, ldB, "B", nullptr, 0, 1, C, ldC, alpha, beta, stream, st);
     }
   }
   constexpr int kBoxN = kPair ? T2::kBNHalf : T1::kBN;
@@ -979,13 +978,12 @@ bool small_group_ok(int n, int group_size, int b) {
 // Up to two tiles per SM otherwise only as long as there is little to do (2000 tile steps, about 7 us): it rotates X for
 // each of its narrow tiles.  us against the best other route: 3332 x 896 x 464 b 16 14.6 / 16.9, 3967 x 704 x 696 b 8 23.2 / 23.2, 3967 x
 // 896 x 1472 b 8 31.8 / 25.2; with unaligned rows of C 2802 x 1453 x 776 b 8 27.3 / 28.1, 556 x 5034 x 3104 b 32 47.9 / 34.
-bool small_oft_wins(int m, int n, int k, int b, int pieces, bool aligned, const DeviceState* st) {
+bool small_oft_wins(const SmallPlan& p, int m, int n, int k, int b, int pieces, bool aligned, const DeviceState* st) {
   const long long t128 = tiles_128(m, n), pairs = st->sm_count / 2;
   const int steps = (k + 63) / 64;
   if (t128 > 2ll * st->sm_count) return false;
   if (t128 > st->sm_count && (aligned ? t128 * steps <= 2000 : steps <= 16)) return true;
   if (t128 > st->sm_count && m > 128) return false;
-  const SmallPlan p = small_plan(small_oft_kind(b), n, m, k, st);
   const long long ctas = t128 * pieces, t256 = ((static_cast<long long>(m) + 255) / 256) * ((static_cast<long long>(n) + 255) / 256);
   const double step = b == 128 ? 0.6 : (p.two && ctas > st->sm_count ? 0.66 : 0.47);
   const double small = 6.0 + static_cast<double>((ctas + p.slots - 1) / p.slots) * steps / pieces * step;
@@ -997,9 +995,12 @@ bool small_oft_wins(int m, int n, int k, int b, int pieces, bool aligned, const 
 // alone (not by where a part's C lies, and not for a slab that is one small group by itself of a whole whose groups the
 // kernel cannot take); with K whole, the kernel has the bits of every other route and each part may choose for itself.
 bool oft_takes_small(const Whole& w, int m, int n, int group_size, int k, int b, bool aligned, const DeviceState* st, int* pieces) {
-  *pieces = small_group_ok(w.n, w.group_size, b) ? small_pieces(small_oft_kind(b), w.n, w.m, k, st) : 1;
-  if (*pieces > 1) return small_oft_wins(w.m, w.n, k, b, *pieces, true, st);
-  return small_group_ok(n, group_size, b) && small_oft_wins(m, n, k, b, 1, aligned, st);
+  const SmallKind kind = small_oft_kind(b);
+  const SmallPlan wp = small_plan(kind, w.m, k, st);
+  *pieces = small_group_ok(w.n, w.group_size, b) ? small_pieces(kind, wp, w.n, w.m) : 1;
+  if (*pieces > 1) return small_oft_wins(wp, w.m, w.n, k, b, *pieces, true, st);
+  const SmallPlan p = w.m == m ? wp : small_plan(kind, m, k, st);  // the plan is one of the rows of X
+  return small_group_ok(n, group_size, b) && small_oft_wins(p, m, n, k, b, 1, aligned, st);
 }
 
 // Groups wide enough for the kernels that share one X.R per row block among N tiles.
@@ -1010,7 +1011,8 @@ int choose_route(int m, int n, int group_size, int k, int b, bool aligned, const
   int path = g_oft_path != 0 ? g_oft_path : opt(kOptOftRoute);
   const bool can_share = kOftPair && st->pool != nullptr;  // routes 2, 3 and 4 need scratch from the pool
   const Whole w = g_whole.m > 0 ? g_whole : Whole{m, n, group_size};
-  *pieces = path == 5 && small_group_ok(w.n, w.group_size, b) ? small_pieces(small_oft_kind(b), w.n, w.m, k, st) : 1;
+  *pieces = 1;
+  if (path == 5 && small_group_ok(w.n, w.group_size, b)) *pieces = small_pieces(small_oft_kind(b), small_plan(small_oft_kind(b), w.m, k, st), w.n, w.m);
   if (path == 2 || path == 3 || path == 4 || path == 5) return can_share ? path : 1;
   if (path == 1 || !can_share) return 1;
   if (opt(kOptSmallTiles) != 0 && oft_takes_small(w, m, n, group_size, k, b, aligned, st, pieces)) return 5;
@@ -1064,7 +1066,7 @@ int launch_oft(int m, int n, int k, int group_size, const void* A, int ldA, cons
   if constexpr (kOftPair) {
     if (route == 5 && small_group_ok(n, group_size, kB)) {
       using TS = SmallTraits<__half, __half, false, kB>;
-      return launch_small<TS>(pieces, n, m, k, B, ldB, "B", A, ldA, "A", R, ldR, group_size, C, ldC, 1.f, 0.f, stream, st);
+      return launch_small<TS>(small_plan(small_kind<TS>(), m, k, st), pieces, n, m, k, B, ldB, "B", A, ldA, "A", R, ldR, group_size, C, ldC, 1.f, 0.f, stream, st);
     }
     if ((route == 3 || route == 4) && (group_size == n || group_size % kBN == 0)) {
       const int rc = oft_ring<kB>(m, n, k, group_size, A, ldA, B, ldB, R, ldR, C, ldC, stream, st, route == 4);
