@@ -552,8 +552,8 @@ int launch_gemm_bn(int m, int n, int k, const void* A, int ldA, const void* B, i
       }
     }
     const long long tiles = static_cast<long long>((m + 2 * T2::kBM - 1) / (2 * T2::kBM)) * ((n + T2::kBN - 1) / T2::kBN);
-    // Split along K for problems of at most half a wave of tiles (those small_kernel does not take: a second operand
-    // pair).  With P SM pairs and T <= P / 2 tiles, every
+    // Split along K for products with a second operand pair of at most half a wave of tiles (small_kernel takes all others
+    // of that size: P / 2 pair tiles are no more than 2 P tiles of 128 x 128).  With P SM pairs and T <= P / 2 tiles, every
     // tile is cut into s = P / T pieces along K (at most 4, at least 8 K steps each) that run on otherwise idle
     // pairs and are summed by whichever piece of a tile finishes last (fp32 partial tiles in pool scratch, summed
     // in piece order: deterministic; no CTA waits for another).  Measured: M = N = 1024, K = 8192 fp16 49 -> 37 us.
@@ -563,36 +563,39 @@ int launch_gemm_bn(int m, int n, int k, const void* A, int ldA, const void* B, i
     const long long all_pairs = st->sm_count / 2;
     const long long full_waves = tiles / all_pairs, rest = tiles % all_pairs;
     const long long k_steps_all = (k + T2::kBK - 1) / T2::kBK + (k2 + T2::kBK - 1) / T2::kBK;
-    long long parts = (rest > 0 && rest * 2 <= all_pairs && full_waves == 0 && !big && st->pool) ? all_pairs / rest : 1;
+    long long parts = (k2 > 0 && rest > 0 && rest * 2 <= all_pairs && full_waves == 0 && !big && st->pool) ? all_pairs / rest : 1;
     if (parts > 4) parts = 4;
     if (parts > k_steps_all / 8) parts = k_steps_all / 8;
-    if (opt(kOptGemmSplit) == 0 || g_whole_k || alpha != 1.f || beta != 0.f) parts = 1;  // the split instance sums pieces, it does not scale
-    if (parts >= 2) {
-      void* scratch = nullptr;
-      const size_t tile_floats = static_cast<size_t>(T2::kBM) * T2::kBN;
-      const size_t count_bytes = (static_cast<size_t>(rest) * 2 * sizeof(int) + 255) & ~static_cast<size_t>(255);
-      const size_t bytes = count_bytes + static_cast<size_t>(rest) * parts * 2 * tile_floats * sizeof(float);
-      if (cudaMallocFromPoolAsync(&scratch, bytes, st->pool, stream) == cudaSuccess) {
-        CUDA_TRY(cudaMemsetAsync(scratch, 0, count_bytes, stream));
-        args.split_first = static_cast<unsigned>(tiles - rest);
-        args.split_parts = static_cast<int>(parts);
-        args.split_count = static_cast<int*>(scratch);
-        args.split_scratch = reinterpret_cast<float*>(static_cast<unsigned char*>(scratch) + count_bytes);
-        auto kernel = gemm2_kernel<T2, true>;
-        if (int rc = opt_in_smem(kernel, T2::kSmemBytes)) {
+    if (opt(kOptGemmSplit) == 0 || alpha != 1.f || beta != 0.f) parts = 1;  // the split instance sums pieces, it does not scale
+    constexpr bool kSecondPair = !kNT && std::is_same<TIn, __half>::value && std::is_same<TOut, __half>::value;  // what takes one
+    if constexpr (kSecondPair) {
+      if (parts >= 2) {
+        void* scratch = nullptr;
+        const size_t tile_floats = static_cast<size_t>(T2::kBM) * T2::kBN;
+        const size_t count_bytes = (static_cast<size_t>(rest) * 2 * sizeof(int) + 255) & ~static_cast<size_t>(255);
+        const size_t bytes = count_bytes + static_cast<size_t>(rest) * parts * 2 * tile_floats * sizeof(float);
+        if (cudaMallocFromPoolAsync(&scratch, bytes, st->pool, stream) == cudaSuccess) {
+          CUDA_TRY(cudaMemsetAsync(scratch, 0, count_bytes, stream));
+          args.split_first = static_cast<unsigned>(tiles - rest);
+          args.split_parts = static_cast<int>(parts);
+          args.split_count = static_cast<int*>(scratch);
+          args.split_scratch = reinterpret_cast<float*>(static_cast<unsigned char*>(scratch) + count_bytes);
+          auto kernel = gemm2_kernel<T2, true>;
+          if (int rc = opt_in_smem(kernel, T2::kSmemBytes)) {
+            cudaFreeAsync(scratch, stream);
+            release_round_counters(st, stream, rounds);
+            return rc;
+          }
+          const long long items = tiles - rest + rest * parts;
+          const int pairs = static_cast<int>(items < all_pairs ? items : all_pairs);
+          const cudaError_t launched = launch_dependent(kernel, 2 * pairs, T2::kThreads, T2::kSmemBytes, stream, ma, mb, ma2, mb2, args);
           cudaFreeAsync(scratch, stream);
           release_round_counters(st, stream, rounds);
-          return rc;
+          CUDA_TRY(launched);
+          return B200_OK;
         }
-        const long long items = tiles - rest + rest * parts;
-        const int pairs = static_cast<int>(items < all_pairs ? items : all_pairs);
-        const cudaError_t launched = launch_dependent(kernel, 2 * pairs, T2::kThreads, T2::kSmemBytes, stream, ma, mb, ma2, mb2, args);
-        cudaFreeAsync(scratch, stream);
-        release_round_counters(st, stream, rounds);
-        CUDA_TRY(launched);
-        return B200_OK;
+        cudaGetLastError();  // no scratch: the plain schedule
       }
-      cudaGetLastError();  // no scratch: the plain schedule
     }
     auto kernel = gemm2_kernel<T2>;
     if (int rc = opt_in_smem(kernel, T2::kSmemBytes)) return rc;

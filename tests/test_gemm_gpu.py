@@ -192,6 +192,37 @@ def test_gemm_second_operand_pair(lib, cuda, pair_build, m, n, k, k2):
     assert np.all(np.abs(got.astype(np.float64) - ref) <= 2e-3 * (np.abs(ref) + 1))
 
 
+@pytest.mark.parametrize("m,n,k,k2", [(200, 328, 1544, 64), (512, 768, 1024, 1096), (136, 1000, 8, 2048)])
+def test_gemm_second_operand_pair_cut_along_k(lib, cuda, pair_build, m, n, k, k2):
+    """Few tiles and a long K: the pair kernel cuts K into pieces (three or four here, one across the seam of the two operand
+    pairs) and adds up their fp32 tiles.  Cut or whole, a result is one rounding to half away from fp32 sums of K / 16 MMAs,
+    each of which loses at most 2^-23 of the sum so far; with operands of U(-1, 1) that sum stays below 8 standard
+    deviations, 8 K^(1/2) / 3."""
+    if not pair_build:
+        pytest.skip("the second operand pair is a feature of the CTA-pair kernel")
+    import torch
+
+    rng = np.random.default_rng(14)
+    A, B, A2, B2 = (rng.uniform(-1, 1, (r, c)).astype(np.float16) for r, c in ((m, k), (n, k), (m, k2), (n, k2)))
+    dA, dB, dA2, dB2 = (torch.from_numpy(x).to(cuda) for x in (A, B, A2, B2))
+
+    def run(split):
+        dC = torch.full((n + 1, m + 3), -7.0, dtype=torch.float16, device=cuda)
+        with ops.option("gemm_split", split, lib):
+            ops.gemm_tn_acc2(m, n, k, dA, k, dB, k, k2, dA2, k2, dB2, k2, dC, m + 3, lib=lib)
+        assert ops.device_status(lib)[0] == 0
+        out = dC.cpu().numpy()
+        assert np.all(out[n] == -7.0) and np.all(out[:, m:] == -7.0)
+        return out[:n, :m].T.astype(np.float64)
+
+    cut, whole = run(-1), run(0)
+    assert np.array_equal(cut, run(-1))
+    ref = A.astype(np.float64) @ B.astype(np.float64).T + A2.astype(np.float64) @ B2.astype(np.float64).T
+    bound = (k + k2) / 16 * 2.0 ** -23 * 8 / 3 * (k + k2) ** 0.5
+    for got in (cut, whole):
+        assert np.all(np.abs(got - ref) <= 2.0 ** -11 * (np.abs(ref) + bound) + bound), float(np.abs(got - ref).max())
+
+
 @pytest.mark.parametrize("m,n,k,r", [(256, 512, 256, 16), (200, 328, 192, 64), (1024, 1024, 512, 8), (128, 256, 128, 0)])
 def test_lora_matches_three_gemm_arithmetic(lib, cuda, pair_build, m, n, k, r):
     if not pair_build and r > 0:
