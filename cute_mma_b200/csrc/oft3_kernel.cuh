@@ -287,14 +287,14 @@ oft3_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
           const uint64_t r_desc = r_desc0 + static_cast<uint64_t>(s * (T::kS1Bytes >> 4));
           if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < T::kBK / 16; ++kk) {
-            // b < 64: the stage holds 64/b diagonal blocks; slice kk belongs to block (kk*16)/b and lands in
-            // columns [blk*b, blk*b+b).  b >= 64: one block, accumulated over the unit.
-            constexpr bool small = T::kB < 64;
-            const int blk = small ? (kk * 16) / T::kB : 0;
-            const uint32_t accum = small ? ((((kk * 16) % T::kB) != 0) ? 1u : 0u) : ((su > 0 || kk > 0) ? 1u : 0u);
-            umma_f16_ss_pair(d1 + blk * T::kB, x_desc + kk * 2, r_desc + kk * 2, idesc1, accum);
-          }
+            for (int kk = 0; kk < T::kBK / 16; ++kk) {
+              // b < 64: the stage holds 64/b diagonal blocks; slice kk belongs to block (kk*16)/b and lands in
+              // columns [blk*b, blk*b+b).  b >= 64: one block, accumulated over the unit.
+              constexpr bool small = T::kB < 64;
+              const int blk = small ? (kk * 16) / T::kB : 0;
+              const uint32_t accum = small ? ((((kk * 16) % T::kB) != 0) ? 1u : 0u) : ((su > 0 || kk > 0) ? 1u : 0u);
+              umma_f16_ss_pair(d1 + blk * T::kB, x_desc + kk * 2, r_desc + kk * 2, idesc1, accum);
+            }
             umma_commit_pair(empty1 + 8 * s, 3);
             if (su == T::kStagesPerUnit - 1) umma_commit_pair(x_acc + 8 * xb, 3);  // the rotation epilogues of both CTAs start on their halves
           }
@@ -351,7 +351,7 @@ oft3_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
             ++tcount;
           }
         }
-      phase ^= 1;
+        phase ^= 1;
       }
     }
     __syncwarp();
@@ -488,27 +488,13 @@ oft3_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
       }
       if (args.n_more > 0) {
         // Further destinations (other GPUs' memory): a write of 16 bytes per lane, each to another row, crosses
-        // NVLink as 32 small packets.  The warp's 32 rows x 128 bytes are therefore transposed in registers first
-        // (butterfly of lane exchanges, 32 x 32 words at a time), after which the 32 lanes write the 128 contiguous
-        // bytes of one row with one instruction.  Needs 4-byte aligned rows; else the row-per-lane stores.
+        // NVLink as 32 small packets.  The warp's 32 rows x 128 bytes are therefore transposed in registers first, after
+        // which the 32 lanes write the 128 contiguous bytes of one row with one instruction.  Needs 4-byte aligned rows;
+        // else the row-per-lane stores.
         bool words = (args.ldC & 1) == 0;
         for (int d = 0; d < args.n_more; ++d) words = words && (reinterpret_cast<uintptr_t>(args.C_more[d]) & 3) == 0;
         if (words) {
-#pragma unroll
-          for (int blk = 0; blk < T::kBN / 64; ++blk) {
-#pragma unroll
-            for (int sft = 16; sft >= 1; sft >>= 1) {
-              const bool upper = (lane & sft) != 0;
-#pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                if (j & sft) continue;
-                uint32_t& lo = p[blk * 32 + j];
-                uint32_t& hi = p[blk * 32 + j + sft];
-                const uint32_t got = __shfl_xor_sync(0xFFFFFFFFu, upper ? lo : hi, sft);
-                if (upper) lo = got; else hi = got;
-              }
-            }
-          }
+          warp_transpose_words<T::kBN / 64>(p, lane);
           // now p[blk * 32 + i] of lane L is word (blk * 32 + L) of row i of this warp
           const int row0 = tm * 2 * T::kBM + rank * T::kBM + quad * 32;
           for (int d = 0; d < args.n_more; ++d) {

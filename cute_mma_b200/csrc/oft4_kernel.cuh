@@ -173,14 +173,14 @@ __device__ __forceinline__ bool oft4_rotate(int warp, int lane, uint32_t rank, B
           const uint64_t r_desc = r_desc0 + static_cast<uint64_t>(s * (T::kS1Bytes >> 4));
           if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < T::kBK / 16; ++kk) {
-            // b < 64: the stage holds 64/b diagonal blocks; slice kk belongs to block (kk*16)/b and lands in
-            // columns [blk*b, blk*b+b).  b >= 64: one block, accumulated over the unit.
-            constexpr bool small = T::kB < 64;
-            const int blk = small ? (kk * 16) / T::kB : 0;
-            const uint32_t accum = small ? ((((kk * 16) % T::kB) != 0) ? 1u : 0u) : ((su > 0 || kk > 0) ? 1u : 0u);
-            umma_f16_ss_pair(d1 + blk * T::kB, x_desc + kk * 2, r_desc + kk * 2, idesc1, accum);
-          }
+            for (int kk = 0; kk < T::kBK / 16; ++kk) {
+              // b < 64: the stage holds 64/b diagonal blocks; slice kk belongs to block (kk*16)/b and lands in
+              // columns [blk*b, blk*b+b).  b >= 64: one block, accumulated over the unit.
+              constexpr bool small = T::kB < 64;
+              const int blk = small ? (kk * 16) / T::kB : 0;
+              const uint32_t accum = small ? ((((kk * 16) % T::kB) != 0) ? 1u : 0u) : ((su > 0 || kk > 0) ? 1u : 0u);
+              umma_f16_ss_pair(d1 + blk * T::kB, x_desc + kk * 2, r_desc + kk * 2, idesc1, accum);
+            }
             umma_commit_pair(sm.empty1 + 8 * s, 3);
             if (su == T::kStagesPerUnit - 1) umma_commit_pair(sm.x_acc + 8 * buf, 3);  // the rotation epilogues of both CTAs start on their halves
           }
@@ -429,7 +429,7 @@ oft4_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ 
               ++tcount;
             }
           }
-        phase ^= 1;
+          phase ^= 1;
         }
       }
       __syncwarp();

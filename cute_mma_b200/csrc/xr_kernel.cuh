@@ -124,14 +124,14 @@ xr_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CU
           const uint64_t r_desc = r_desc0 + static_cast<uint64_t>(s * (T::kSBytes >> 4));
           if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < T::kBK / 16; ++kk) {
-            // b < 64: the stage holds 64/b diagonal blocks; slice kk belongs to block (kk*16)/b and lands in
-            // columns [blk*b, blk*b+b).  b >= 64: one block, accumulated over the unit.
-            constexpr bool small = T::kB < 64;
-            const int blk = small ? (kk * 16) / T::kB : 0;
-            const uint32_t accum = small ? ((((kk * 16) % T::kB) != 0) ? 1u : 0u) : ((su > 0 || kk > 0) ? 1u : 0u);
-            umma_f16_ss(d + blk * T::kB, a_desc + kk * 2, r_desc + kk * 2, idesc, accum);
-          }
+            for (int kk = 0; kk < T::kBK / 16; ++kk) {
+              // b < 64: the stage holds 64/b diagonal blocks; slice kk belongs to block (kk*16)/b and lands in
+              // columns [blk*b, blk*b+b).  b >= 64: one block, accumulated over the unit.
+              constexpr bool small = T::kB < 64;
+              const int blk = small ? (kk * 16) / T::kB : 0;
+              const uint32_t accum = small ? ((((kk * 16) % T::kB) != 0) ? 1u : 0u) : ((su > 0 || kk > 0) ? 1u : 0u);
+              umma_f16_ss(d + blk * T::kB, a_desc + kk * 2, r_desc + kk * 2, idesc, accum);
+            }
             umma_commit(empty + 8 * s);
             if (su == T::kStagesPerUnit - 1) umma_commit(x_full + 8 * buf);
           }
