@@ -38,6 +38,16 @@ def pair_build(lib):
     return ops.kernel_info(lib)["oft"]["ctas"] == 2
 
 
+@pytest.fixture(params=[-1, 0], ids=["chosen", "no_small_kernel"])
+def small_tiles(request, lib):
+    """The library's own choice of kernel, then the same test without the kernel for small problems, which otherwise takes
+    almost every shape a test can afford."""
+    from cute_mma_b200 import ops
+
+    with ops.option("small_tiles", request.param, lib):
+        yield request.param
+
+
 @pytest.fixture(autouse=True)
 def room_in_the_tensor_cache(request):
     """test_zz_no_alloc compares the driver's free memory around calls that also clone a 1 MB tensor: torch's cache must

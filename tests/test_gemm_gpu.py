@@ -50,6 +50,7 @@ def truth(layout, m, n, k, A, ldA, B, ldB, rows, cols, tf32_mode=0):
 SHAPES = [(128, 256, 64), (128, 256, 512), (384, 512, 256), (200, 328, 136), (72, 40, 64), (640, 1280, 1024)]
 
 
+@pytest.mark.usefixtures("small_tiles")
 @pytest.mark.parametrize("layout", ["TN", "NT"])
 @pytest.mark.parametrize("m,n,k", SHAPES)
 def test_gemm_half_matches_fp64_truth(lib, cuda, layout, m, n, k):
@@ -62,6 +63,7 @@ def test_gemm_half_matches_fp64_truth(lib, cuda, layout, m, n, k):
     assert worst < 2e-3, worst
 
 
+@pytest.mark.usefixtures("small_tiles")
 @pytest.mark.parametrize("layout", ["TN", "NT"])
 @pytest.mark.parametrize("m,n,k", SHAPES)
 def test_gemm_float_tf32_matches_fp64_truth(lib, cuda, layout, m, n, k):
@@ -76,6 +78,7 @@ def test_gemm_float_tf32_matches_fp64_truth(lib, cuda, layout, m, n, k):
     assert bad_t == 0, (bad_t, worst_t)
 
 
+@pytest.mark.usefixtures("small_tiles")
 @pytest.mark.parametrize("layout,dtype", [("TN", "half"), ("NT", "half"), ("TN", "float"), ("NT", "float")])
 def test_gemm_padded_leading_dimensions(lib, cuda, layout, dtype):
     m, n, k = 200, 328, 136
@@ -112,6 +115,7 @@ def test_gemm_dispatcher_and_errors(lib, cuda):
     assert e.value.code == ops.EINVAL
 
 
+@pytest.mark.usefixtures("small_tiles")
 @pytest.mark.parametrize("layout,dtype", [("TN", "half"), ("NT", "half"), ("TN", "float"), ("NT", "float")])
 def test_gemm_rowmajor_is_the_transpose_of_colmajor(lib, cuda, layout, dtype):
     """b200_gemm_rowmajor writes C[i][j] where b200_gemm writes C[i + j*ldC]: same numbers, bit for bit
@@ -135,6 +139,7 @@ def test_gemm_rowmajor_is_the_transpose_of_colmajor(lib, cuda, layout, dtype):
     assert e.value.code == ops.EINVAL
 
 
+@pytest.mark.usefixtures("small_tiles")
 @pytest.mark.parametrize("layout", ["TN", "NT"])
 @pytest.mark.parametrize("in_type,out_type,alpha,beta", [(0, 0, 1.0, 0.0), (0, 0, 0.5, 0.0), (0, 0, -1.25, 0.75), (0, 1, 1.0, 0.0), (0, 1, 2.0, -0.5),
                                                          (2, 1, 1.0, 0.0), (2, 1, 0.25, 1.0)])
@@ -223,6 +228,7 @@ def test_gemm_second_operand_pair_cut_along_k(lib, cuda, pair_build, m, n, k, k2
         assert np.all(np.abs(got - ref) <= 2.0 ** -11 * (np.abs(ref) + bound) + bound), float(np.abs(got - ref).max())
 
 
+@pytest.mark.usefixtures("small_tiles")
 @pytest.mark.parametrize("m,n,k,r", [(256, 512, 256, 16), (200, 328, 192, 64), (1024, 1024, 512, 8), (128, 256, 128, 0)])
 def test_lora_matches_three_gemm_arithmetic(lib, cuda, pair_build, m, n, k, r):
     if not pair_build and r > 0:

@@ -70,6 +70,7 @@ CASES = [
 ]
 
 
+@pytest.mark.usefixtures("small_tiles")
 @pytest.mark.parametrize("m,n,k,b,gs", CASES)
 def test_oft_matches_oracle(lib, cuda, pair_build, m, n, k, b, gs):
     if gs is not None and gs < 256 and not pair_build:
@@ -126,6 +127,7 @@ TWO_PASS_CASES = [
 ]
 
 
+@pytest.mark.usefixtures("small_tiles")
 @pytest.mark.parametrize("m,n,k,b,gs", TWO_PASS_CASES)
 def test_oft_two_pass_matches_oracle_and_fused(lib, cuda, m, n, k, b, gs):
     """Rotation pass + plain GEMM: same tolerances against the oracle as the fused kernel, and the two
@@ -327,6 +329,7 @@ def test_oft_group_size_limits(lib, cuda, pair_build):
         assert e.value.code == ops.EUNSUPPORTED and "group_size" in e.value.message
 
 
+@pytest.mark.usefixtures("small_tiles")
 def test_oft_padded_leading_dimensions(lib, cuda):
     m, n, k, b = 200, 328, 192, 64
     A, R, B = make_oft_case(m, n, k, b, seed=3)
@@ -339,6 +342,7 @@ def test_oft_padded_leading_dimensions(lib, cuda):
     assert np.array_equal(got.view(np.uint16), got2.view(np.uint16))
 
 
+@pytest.mark.usefixtures("small_tiles")
 def test_oft_permutation_blocks_reference_check(lib, cuda):
     """The reference's own correctness protocol (cute_oft_pc.cu:195-236, 334-350): positive inputs,
     permutation blocks, count of elements above 5e-3 relative error must be zero."""
@@ -350,6 +354,7 @@ def test_oft_permutation_blocks_reference_check(lib, cuda):
     assert errors == 0, (errors, worst)
 
 
+@pytest.mark.usefixtures("small_tiles")
 def test_oft_zero_one_init_is_bit_exact(lib, cuda):
     """--01init (cute_oft_pc.cu:202-216): every partial sum is a small integer, exact in fp16 and
     fp32, so the kernel must agree with the oracle bit for bit (K <= 2048 keeps sums <= 2048)."""
@@ -360,6 +365,7 @@ def test_oft_zero_one_init_is_bit_exact(lib, cuda):
     assert np.array_equal(got.view(np.uint16), ref.view(np.uint16))
 
 
+@pytest.mark.usefixtures("small_tiles")
 def test_oft_structured_block_known_answer(lib, cuda):
     """Known-answer block (idea of playgrounds/bd_construct.cu:117-159): with R_math = I + e0 1^T,
     (x R)[q] = x[q] + x[0] per block, so Y = X' W with X' computed in closed form.  A transposed-R
@@ -373,6 +379,7 @@ def test_oft_structured_block_known_answer(lib, cuda):
     assert np.array_equal(got.astype(np.float64), expect)  # integers below 2048: exact
 
 
+@pytest.mark.usefixtures("small_tiles")
 def test_oft_is_deterministic(lib, cuda):
     m, n, k, b = 384, 512, 512, 64
     A, R, B = make_oft_case(m, n, k, b, seed=11)
@@ -499,6 +506,7 @@ def test_oft_large_full_size_sampled_and_routes_agree(lib, cuda, pair_build):
     assert torch.equal(c_auto.view(torch.int16), c_fused.view(torch.int16))
 
 
+@pytest.mark.usefixtures("small_tiles")
 @pytest.mark.parametrize("m,n,k,b,gs,pad", [(200, 328, 192, 64, None, 0), (5000, 512, 256, 32, None, 8), (4200, 512, 128, 8, 256, 0), (4300, 1024, 128, 16, None, 8)])
 def test_host_buffer_entry_point_matches_device_path(lib, cuda, m, n, k, b, gs, pad):
     """b200_oft_tn_f16_host (pageable numpy buffers here; several row chunks when M exceeds 2048, the chunks'
@@ -534,6 +542,7 @@ def test_bounded_wait_reports_and_recovers(lib, cuda):
     assert oft_ok(got, oracle_full(A, R, B, m, n, k, b))[0] == 0
 
 
+@pytest.mark.usefixtures("small_tiles")
 @pytest.mark.parametrize("m,n,k,b,gs", [(384, 512, 512, 64, None), (200, 328, 192, 32, None), (256, 512, 256, 8, 256), (128, 256, 256, 128, None)])
 def test_a_rw_order_matches_oracle(lib, cuda, m, n, k, b, gs):
     """Y = X.(R.W) (cublas_oft.hpp:58-65): the weight transform against its definition, and the product
@@ -669,6 +678,7 @@ def test_oft_ring_route_on_two_streams(lib, cuda, pair_build, route):
     assert torch.equal(c1, alone) and torch.equal(c2, alone)
 
 
+@pytest.mark.usefixtures("small_tiles")
 @pytest.mark.parametrize("m,n,k,b,gs,pad", [(384, 2048, 256, 64, None, 8), (200, 2056, 192, 32, None, 8), (200, 2055, 192, 32, None, 3),
                                             (200, 2056, 192, 32, None, 9), (256, 512, 256, 64, None, 8), (256, 2048, 128, 128, 1024, 8),
                                             (2304, 5120, 256, 64, None, 8)])
