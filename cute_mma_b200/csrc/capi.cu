@@ -327,11 +327,14 @@ thread_local bool g_whole_k = false;
 // 0.72 us per step between them (both operands of a 128-wide tile are read from shared memory at its full rate), plus
 // the fixed costs and 1.5 us of epilogue per round.  1848 x 1488 x 489 half: 8.9 against 12.8 us; 2904 x 960 x 11305: 110
 // against 70 us.
-// With K whole (the passes of oft_two_pass) up to 64 K steps only in the first range: 96 tiles of 64 steps 29.6 against 36.9
-// us on the pair kernel, 128 tiles of 226 steps 97.9 against 85.
+// With K whole (the GEMMs of oft_two_pass, n the rows of X) few rows only, and up to 64 K steps in the first range.  More
+// rows than one tile go either way behind the rotation pass (us on the pair kernel / on this one: 4571 x 4483 x 256 26.7 /
+// 30.0, 852 x 5069 x 2880 41.7 / 27.8); at no more than one tile per SM 96 tiles of 64 steps take 36.9 / 29.6, 128 tiles of
+// 226 steps 85 / 97.9.
 bool small_wins(int m, int n, int steps, bool whole_k, const DeviceState* st) {
   const long long t128 = tiles_128(m, n), pairs = st->sm_count / 2;
-  if (t128 <= st->sm_count) return !whole_k || steps <= 64;
+  if (whole_k && (n > 128 || (t128 <= st->sm_count && steps > 64))) return false;
+  if (t128 <= st->sm_count) return true;
   const long long t256 = ((static_cast<long long>(m) + 255) / 256) * ((static_cast<long long>(n) + 255) / 256);
   const double rounds = static_cast<double>(t128) / (2.0 * st->sm_count);
   const double small = 5.0 + (rounds > 1.0 ? rounds : 1.0) * (0.72 * steps + 1.5);
