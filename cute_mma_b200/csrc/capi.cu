@@ -320,13 +320,13 @@ long long tiles_128(int m, int n) { return ((static_cast<long long>(m) + 127) / 
 thread_local bool g_whole_k = false;
 
 // Whether small_kernel takes a plain m x n product of `steps` K steps (128 bytes of a row each).
-// As long as its 128 x 128 tiles do not outnumber the SMs, always: every one of 150 random shapes of the operator
-// surface ran faster on it than on the pair kernels, by 1.1 to 6.7 times (fixed cost per launch 5 us against 9 to 12 us,
-// and 256 x 256 tiles leave most SMs idle: 640 x 1280 x 1024 TF32 29 -> 10 us).  Above, the two are compared by a model
-// fitted to 120 random shapes: a round of pair tiles costs 0.36 us per K step on 74 pairs, two small tiles per SM cost
-// 0.72 us per step between them (both operands of a 128-wide tile are read from shared memory at its full rate), plus
-// the fixed costs and 1.5 us of epilogue per round.  1848 x 1488 x 489 half: 8.9 against 12.8 us; 2904 x 960 x 11305: 110
-// against 70 us.
+// As long as its 128 x 128 tiles do not outnumber the SMs, always (fixed cost per launch 5 us against 9 to 12 us, and 256 x
+// 256 tiles leave most SMs idle: 640 x 1280 x 1024 TF32 29 -> 10 us).  Above, the two are compared by a model fitted to 120
+// random shapes: a round of pair tiles costs 0.36 us per K step on 74 pairs, two small tiles per SM cost 0.72 us per step
+// between them (both operands of a 128-wide tile are read from shared memory at its full rate), plus the fixed costs and 1.5
+// us of epilogue per round.  1848 x 1488 x 489 half: 8.9 against 12.8 us; 2904 x 960 x 11305: 110 against 70 us.  On 12 of the
+// 120 it names the slower kernel, by up to 1.16 times where that is this one and 1.32 where it is the pair kernel, whose fixed
+// cost was fitted before its launch became a dependent one (2 us less).
 // With K whole (the GEMMs of oft_two_pass, n the rows of X) few rows only, and up to 64 K steps in the first range.  More
 // rows than one tile go either way behind the rotation pass (us on the pair kernel / on this one: 4571 x 4483 x 256 26.7 /
 // 30.0, 852 x 5069 x 2880 41.7 / 27.8); at no more than one tile per SM 96 tiles of 64 steps take 36.9 / 29.6, 128 tiles of
@@ -390,7 +390,8 @@ SmallPlan small_plan(const SmallKind& kind, int n, int k, const DeviceState* st)
   return p;
 }
 // Pieces along K of an m x n product: as many as there is room for CTAs at once; at least four K steps each, and none
-// below 16 steps (a K loop of 16 steps takes about 4 us, adding up the pieces 1.5).
+// below 16 steps (a K loop of 16 steps takes about 4 us, adding up the pieces 1.5).  Near that line cutting need not pay:
+// half 640 x 1280 x 1024 takes 8.4 us whole and 9.2 in four pieces; 256 x 256 x 16384 takes 68 whole and 15 in eight.
 int small_pieces(const SmallKind& kind, const SmallPlan& p, int m, int n) {
   const long long tiles = tiles_128(m, n);
   int split = 1;
@@ -1025,10 +1026,12 @@ int choose_route(int m, int n, int group_size, int k, int b, bool aligned, const
   const int k_steps = (k + 63) / 64;
   const bool wide = wide_group(group_size, b);
   // Rotation pass + plain GEMM (route 2).  Rows of C that are not 16-byte aligned and one group: the fused kernels store
-  // them a row at a time after a transpose in registers (route 1) or element by element (route 3); us on routes 1 / 2 / 3: 12375 x 1473 x
-  // 576 b 64 74.6 / 49.2 / 287, 2988 x 4253 x 4176 b 8 125 / 99 / 215, 39866 x 647 x 3456 b 128 254 / 260 / 298.  Short K, a wide
-  // group and more tiles than SM pairs: 16589 x 4904 x 384 b 128 114 / 82 / 140 (route 4 140), 6503 x 7008 x 512 b 64 68 / 56 / 86; with one
-  // round of tiles there is nothing to serialise the rotation with (647 x 4096 x 512 b 64 14.8 / 21.2 / 21.8).
+  // them a row at a time after a transpose in registers (route 1) or element by element (route 3); us on routes 1 / 2 / 3:
+  // 12375 x 1473 x 576 b 64 74.6 / 49.2 / 287, 2988 x 4253 x 4176 b 8 125 / 99 / 215, 39866 x 647 x 3456 b 128 254 / 260 / 298 (level
+  // with route 1 where the group is narrow and K long).  Short K, a wide group and more tiles than SM pairs: 16589 x 4904 x
+  // 384 b 128 114 / 82 / 140 (route 4 140), 6503 x 7008 x 512 b 64 68 / 56 / 86; with one round of tiles there is nothing to
+  // serialise the rotation with (647 x 4096 x 512 b 64 14.8 / 21.2 / 21.8).  Few rows of X: the GEMM runs on small_kernel, 1 x
+  // 131072 x 448 b 64 38 / 29 / 44.
   const bool group_ok = group_size == n || group_size % static_cast<int>(CurrCompParams::bN) == 0;  // what the fused routes take of these widths
   if (g_more.n == 0 && group_ok && two_pass_fits(k)) {
     if (!aligned && group_size == n) return 2;
@@ -1037,10 +1040,10 @@ int choose_route(int m, int n, int group_size, int k, int b, bool aligned, const
   }
   if (!wide) return 1;
   if (g_more.n > 0) return 3;  // of the ring kernels, only oft3_kernel stores to further destinations
-  // Route 4 also wants long tiles: its product pairs write C with the plain GEMM's epilogue (one 2-byte store per
-  // element), which must fit beside a tile's MMAs.  Interleaved runs, route 4 / route 3 time: M 32768, N 28672, K 1024,
-  // b 64: 1.61; M 262144, N 12288, K 2048, b 64 (3 pairs): 1.05; M 65536, N 28672, b 128 (2 pairs), K 2048: 0.86,
-  // K 4096: 0.88.
+  // Route 4 also wants long tiles: its product pairs write C with the plain GEMM's epilogue, which must fit beside a tile's
+  // MMAs.  The line was drawn when that epilogue took 16 instructions per column (route 4 / route 3 time: M 32768, N 28672, K
+  // 1024, b 64: 1.61; M 262144, N 12288, K 2048, b 64, 3 pairs: 1.05).  It takes four since, and the same shapes now
+  // measure 0.66 and 0.84, 3001 x 11008 x 4096 b 32 (4 pairs) 0.95; M 65536, N 28672, K 2048, b 128 (2 pairs) 0.77.
   const RingPlan p = ring_plan(m, group_size, k, st);
   const bool split = p.rot_pairs >= 1 && p.rot_pairs <= 3 && k_steps >= 32 && (p.rot_pairs <= 2 || k_steps >= 64);
   return split ? 4 : 3;

@@ -10,8 +10,9 @@
 //   * the tiles are cut along K into `split` pieces (the CTAs of one cluster), so that every SM streams part of P;
 //     the pieces' fp32 partial tiles meet in distributed shared memory, summed in piece order by the CTA that owns
 //     the columns: no scratch in global memory, no counters, the same bits on every run,
-//   * CTAs hold at most half of an SM (shared memory and tensor memory), so two are resident and one's prologue and
-//     epilogue run under the other's main loop.
+//   * CTAs hold half of an SM's tensor memory and, where a ring of the least depth fits, half of its shared memory: plain
+//     products always, rotated ones with tiles of at most 80 columns (48 with 64 x 64 blocks, never with 128 x 128).  Two
+//     are resident then, and one's prologue and epilogue run under the other's main loop.
 // Bound: small M reads P once from HBM (8 x 4096 x 4096: 33.5 MB); the rest is launch and pipeline latency.
 //
 // Roles (256 threads): warp 0 TMA producer, warp 1 issues the product, warp 2 owns tensor memory, warp 3 issues the

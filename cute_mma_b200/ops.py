@@ -124,8 +124,9 @@ def oft_tn(m, n, k, A, ldA, B, ldB, R, ldR, C, ldC, stream=None, *, group_size=N
 
 
 def oft_tn_two_pass(m, n, k, A, ldA, B, ldB, R, ldR, C, ldC, stream=None, *, group_size=None, reconn_sz=8, lib=None) -> None:
-    """oft_tn as a rotation pass (X.R written once to device scratch) followed by the plain GEMM, the route
-    oft_tn takes by itself when a group spans many N tiles (see b200_oft_tn_f16_two_pass in the header)."""
+    """oft_tn as a rotation pass (X.R written once to device scratch) followed by the plain GEMM, the route oft_tn takes by
+    itself for short K in wide groups and for one group with unaligned rows of C (see b200_oft_tn_f16_two_pass in the
+    header)."""
     lib = lib or load_library()
     gs = n if group_size is None else group_size
     _check(lib, lib.b200_oft_tn_f16_two_pass(m, n, k, gs, reconn_sz, _ptr(A), ldA, _ptr(B), ldB, _ptr(R), ldR, _ptr(C), ldC, _stream(stream)))

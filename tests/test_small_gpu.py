@@ -1,4 +1,4 @@
-"""small_kernel (problems with no more 128 x 128 tiles than SMs) at the edges of its tiles, its pieces along K and its
+"""small_kernel (problems of up to about one 128 x 128 tile per SM) at the edges of its tiles, its pieces along K and its
 rotation buffers, against the routes it replaces (bit for bit where K is not cut) and against fp64."""
 import numpy as np
 import pytest
