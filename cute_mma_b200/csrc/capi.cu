@@ -23,6 +23,7 @@
 #include "oft_config.hpp"
 #include "gemm_kernel.cuh"
 #include "gemm2_kernel.cuh"
+#include "gemm2w_kernel.cuh"
 #include "oft_kernel.cuh"
 #include "oft2_kernel.cuh"
 #include "xr_kernel.cuh"
@@ -51,7 +52,7 @@ int fail(int code, const char* fmt, ...) {
 // library choose".  The B200_* environment variables of the same meaning are read ONCE, at the first use
 // of any option in the process, as initial values; after that only b200_set_option changes them, so
 // nothing on the launch path reads the environment.
-enum OptionId { kOptOftRoute, kOptRaster, kOptTileSync, kOptL2Hints, kOptGemmTileSync, kOptGemmL2Hints, kOptGemmSplit, kOptMaps3d, kOptRingBands, kOptPrefetch, kOptRotPairs, kOptSmallTiles, kOptSmallSplit, kOptPdl, kOptSmallStages, kOptCount };
+enum OptionId { kOptOftRoute, kOptRaster, kOptTileSync, kOptL2Hints, kOptGemmTileSync, kOptGemmL2Hints, kOptGemmSplit, kOptMaps3d, kOptRingBands, kOptPrefetch, kOptRotPairs, kOptSmallTiles, kOptSmallSplit, kOptPdl, kOptSmallStages, kOptGemmWide, kOptCount };
 struct OptionDef { const char* name; const char* env; int initial; };
 constexpr OptionDef kOptionDefs[kOptCount] = {
     {"oft_route", "B200_OFT_PATH", 0},            // 0 choose, 1 X.R in tensor memory per tile, 2 two passes, 3 / 4 X.R shared through the L2 ring
@@ -69,6 +70,7 @@ constexpr OptionDef kOptionDefs[kOptCount] = {
     {"small_split", "B200_SMALL_SPLIT", -1},      // small-problem kernel: pieces along K (1..8)
     {"pdl", "B200_PDL", -1},                      // 0: no programmatic dependent launch
     {"small_stages", "B200_SMALL_STAGES", -1},    // small-problem kernel: ring depth
+    {"gemm_wide", "B200_GEMM_WIDE", -1},          // plain GEMM: 0 never tiles of 256 x 512, 1 always
 };
 std::atomic<int> g_opt[kOptCount];
 std::once_flag g_opt_once;
@@ -185,14 +187,6 @@ int make_map(CUtensorMap* map, const void* base, int elem_bytes, long long inner
                         atom32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(B200_ECUDA, "%s: cuTensorMapEncodeTiled failed with CUresult %d", what, static_cast<int>(r));
   return B200_OK;
-}
-
-// Tile order of a launch.  The "raster" option overrides it for experiments.
-int raster_for(long long operand_bytes, bool oft) {
-  if (opt(kOptRaster) >= 0) return opt(kOptRaster);
-  // Bands of 8 tile rows for the fused kernel once the operands no longer sit in L2 beside each other (see
-  // launch_oft_gt); the plain GEMM chooses its order in launch_gemm_bn.
-  return (oft && operand_bytes > (40ll << 20)) ? 8 : 0;
 }
 
 // 3-D map over an MN-major matrix [outer = K rows][inner = MN contiguous], inner a multiple of `chunk`:
@@ -320,13 +314,14 @@ long long tiles_128(int m, int n) { return ((static_cast<long long>(m) + 127) / 
 thread_local bool g_whole_k = false;
 
 // Whether small_kernel takes a plain m x n product of `steps` K steps (128 bytes of a row each).
-// As long as its 128 x 128 tiles do not outnumber the SMs, always (fixed cost per launch 5 us against 9 to 12 us, and 256 x
-// 256 tiles leave most SMs idle: 640 x 1280 x 1024 TF32 29 -> 10 us).  Above, the two are compared by a model fitted to 120
-// random shapes: a round of pair tiles costs 0.36 us per K step on 74 pairs, two small tiles per SM cost 0.72 us per step
-// between them (both operands of a 128-wide tile are read from shared memory at its full rate), plus the fixed costs and 1.5
-// us of epilogue per round.  1848 x 1488 x 489 half: 8.9 against 12.8 us; 2904 x 960 x 11305: 110 against 70 us.  On 12 of the
-// 120 it names the slower kernel, by up to 1.16 times where that is this one and 1.32 where it is the pair kernel, whose fixed
-// cost was fitted before its launch became a dependent one (2 us less).
+// As long as its 128 x 128 tiles do not outnumber the SMs, always (fixed cost per launch 5 us against 7 to 9 us, and 256 x
+// 256 tiles leave most SMs idle: 640 x 1280 x 1024 TF32 29 -> 10 us), and for n <= 128, of which a pair tile covers twice
+// the columns at least (65536 x 120 x 4096 half 100 against 128 us, 131072 x 64 x 512 31 against 40).  Above, the two are
+// compared by a model fitted to 110 random shapes of 149 to 1100 tiles: a K step of two tiles per SM costs 0.74 us per 128
+// columns, a last wave of one tile per SM 0.24 and of more 0.48; a round of pair tiles 0.34 us per step on 74 pairs, either
+// size; plus fixed costs.  What it picks takes 1.2 % longer than the better of the two on average, at worst 14 % (10072 x
+// 181 x 799 NT half 15.2 against 13.4).  5936 x 776 x 5822 NT: 118 against 68 us; 2815 x 6280 x 163: 27 against 20; 11904 x 276 x
+// 263 TF32: 9.9 against 15.7.
 // With K whole (the GEMMs of oft_two_pass, n the rows of X) few rows only, and up to 64 K steps in the first range.  More
 // rows than one tile go either way behind the rotation pass (us on the pair kernel / on this one: 4571 x 4483 x 256 26.7 /
 // 30.0, 852 x 5069 x 2880 41.7 / 27.8); at no more than one tile per SM 96 tiles of 64 steps take 36.9 / 29.6, 128 tiles of
@@ -334,12 +329,25 @@ thread_local bool g_whole_k = false;
 bool small_wins(int m, int n, int steps, bool whole_k, const DeviceState* st) {
   const long long t128 = tiles_128(m, n), pairs = st->sm_count / 2;
   if (whole_k && (n > 128 || (t128 <= st->sm_count && steps > 64))) return false;
-  if (t128 <= st->sm_count) return true;
+  if (t128 <= st->sm_count || n <= 128) return true;
   const long long t256 = ((static_cast<long long>(m) + 255) / 256) * ((static_cast<long long>(n) + 255) / 256);
-  const double rounds = static_cast<double>(t128) / (2.0 * st->sm_count);
-  const double small = 5.0 + (rounds > 1.0 ? rounds : 1.0) * (0.72 * steps + 1.5);
-  const double pair = 11.5 + static_cast<double>((t256 + pairs - 1) / pairs) * (0.36 * steps + 1.5);
+  const long long waves = t128 / (2 * st->sm_count), rest = t128 % (2 * st->sm_count);
+  const int tiles_n = (n + 127) / 128;
+  const double step = (n + tiles_n - 1) / tiles_n / 128.0 * steps;  // K steps of 128 columns
+  const double small = 7.0 + step * (0.74 * waves + (rest == 0 ? 0.0 : rest <= st->sm_count ? 0.24 : 0.48)) + 1.2 * (waves + (rest > 0));
+  const double pair = 8.0 + static_cast<double>((t256 + pairs - 1) / pairs) * (0.34 * steps + 1.4);
   return small < pair;
+}
+
+// Whether the plain GEMM of `steps` K steps runs on tiles of 256 x 512 (gemm2w_kernel).  Both kernels give the longest pair the
+// same number of 256-column tiles, `rounds`; the wide one moves a quarter less between L2 and the SMs and starts with bigger
+// loads, so it needs a second round to pair up and some work to make up for the start.  us on tiles of 256 / 512, 64 random
+// shapes: 12800 x 1123 x 2686 TN 82 / 82, 8192^3 864 / 842, 4690 x 9804 x 9607 NT 906 / 782, TF32 NT 5933 x 7743 x 6727 1331 / 1000;
+// below the lines 1634 x 4191 x 725 TF32 TN (46 K steps in a row) 25 / 26.5, 1296 x 9592 x 349 NT (24) 24.7 / 25.6, above them
+// 3257 x 3051 x 1588 (75) 38.8 / 37.2, NT 12072 x 776 x 421 (21) 23.4 / 21.1, 9304 x 808 x 1265 (40) 29.2 / 27.2.
+bool wide_wins(int m, int n, int steps, bool nt, const DeviceState* st) {
+  const long long pairs = st->sm_count / 2, tiles = static_cast<long long>((m + 255) / 256) * ((n + 255) / 256), rounds = (tiles + pairs - 1) / pairs;
+  return n > 256 && rounds >= 2 && rounds * steps >= (nt ? 40 : 60);
 }
 
 // What the geometry of a launch depends on beside the sizes: an instance of small_kernel.
@@ -482,6 +490,39 @@ int launch_gemm(int m, int n, int k, const void* A, int ldA, const void* B, int 
   return launch_gemm_bn<TIn, TOut, kNT, P, P::bN>(m, n, k, A, ldA, B, ldB, C, ldC, stream_v, k2, A2, ldA2, B2, ldB2, alpha, beta);
 }
 
+// Tile order of the wide kernel: bands of 16 rows of tiles.  The 74 tiles of a round then cover about 4096 x 2368 of C, whose
+// operands are what L2 has to hand out (bands of 8: 2048 x 4736; 8192^3 half 856 us in bands of 8, 849 of 12, 843 of 16, 861 of
+// 32).  The phase lock of the tile rounds (see launch_oft_gt) only pays when the operands are several times L2: 28672 x 16384
+// x 8192 half 6579 us without, 5985 with it; 8192^3 839 / 843, 14959 x 12569 x 274 TF32 287 / 302.  L2 eviction priorities as
+// gemm2_kernel's gain nothing with these bands (5964 / 5985 us without / with them).
+template <class T>
+int launch_wide(int m, int n, int k, const CUtensorMap& ma, const CUtensorMap& mb, int a3d, int b3d, void* C, int ldC, float alpha, float beta,
+                long long operand_bytes, cudaStream_t stream, DeviceState* st) {
+  const int raster = opt(kOptRaster) >= 0 ? opt(kOptRaster) : 16;
+  const int tile_sync = opt(kOptGemmTileSync) >= 0 ? opt(kOptGemmTileSync) : (operand_bytes > 3 * st->l2_bytes ? 1 : 0);
+  const int h = opt(kOptGemmL2Hints);
+  auto kernel = gemm2w_kernel<T>;
+  if (int rc = opt_in_smem(kernel, T::kSmemBytes)) return rc;
+  int* rounds = nullptr;
+  if (tile_sync)
+    if (int rc = round_counters(st, stream, &rounds)) return rc;
+  const long long pairs = st->sm_count / 2, tiles_m = (m + 255) / 256, tiles_n = (n + 255) / 256;
+  const unsigned wide = wide_tiles_whole(tiles_m * (tiles_n / 2), tiles_n % 2 ? tiles_m : 0, pairs);
+  Gemm2WArgs args{m, n, k, C, ldC, st->status, raster, tile_sync, rounds, a3d, b3d, h >= 0 ? hint_word(h / 10) : kL2EvictNormal,
+                  h >= 0 ? hint_word(h % 10) : kL2EvictNormal, wide, alpha, beta};
+  const long long items = tiles_m * tiles_n - wide;
+  const int grid = 2 * static_cast<int>(items < pairs ? items : pairs);
+  cudaError_t e = cudaErrorUnknown;
+  if (args.tile_sync && (e = launch_cooperative(kernel, grid, T::kThreads, T::kSmemBytes, stream, ma, mb, args)) != cudaSuccess) {
+    cudaGetLastError();
+    args.tile_sync = 0;
+  }
+  if (!args.tile_sync) e = launch_dependent(kernel, grid, T::kThreads, T::kSmemBytes, stream, ma, mb, args);
+  release_round_counters(st, stream, rounds);
+  CUDA_TRY(e);
+  return B200_OK;
+}
+
 template <typename TIn, typename TOut, bool kNT, class P, int kBN>
 int launch_gemm_bn(int m, int n, int k, const void* A, int ldA, const void* B, int ldB, void* C, int ldC, void* stream_v,
                    int k2, const void* A2, int ldA2, const void* B2, int ldB2, float alpha, float beta) {
@@ -531,14 +572,22 @@ int launch_gemm_bn(int m, int n, int k, const void* A, int ldA, const void* B, i
   // The same three measures already pay when the two operands together exceed one and a half times L2 (one-pass
   // ncu counters, unthrottled launches): 8192^3 fp16 721 -> 689 us and 1.37 -> 0.85 GB of DRAM reads; M 8192,
   // N 4096, K 8192 354 -> 346 us; 4096 x 16384 x 4096 and below: no difference, so they stay on the z-curve.
-  const bool big = kPair && (static_cast<long long>(m) + n) * k * static_cast<long long>(sizeof(TIn)) > 3ll * st->l2_bytes / 2;
+  const long long operand_bytes = (static_cast<long long>(m) + n) * k * static_cast<long long>(sizeof(TIn));
+  if constexpr (kPair && kBN == 256) {
+    using TW = Gemm2WTraits<TIn, TOut, kNT>;
+    const int steps = (k + TW::kBK - 1) / TW::kBK;
+    if (k2 == 0 && steps >= TW::kMinSteps && (opt(kOptGemmWide) < 0 ? wide_wins(m, n, steps, kNT, st) : opt(kOptGemmWide) != 0))
+      return launch_wide<TW>(m, n, k, ma, mb, a3d, b3d, C, ldC, alpha, beta, operand_bytes, stream, st);
+  }
+  const bool big = kPair && operand_bytes > 3ll * st->l2_bytes / 2;
   int tile_sync = big ? 1 : 0;
   if (opt(kOptGemmTileSync) >= 0) tile_sync = kPair ? opt(kOptGemmTileSync) : 0;
   int* rounds = nullptr;
   if (tile_sync)
     if (int rc = round_counters(st, stream, &rounds)) return rc;
-  int raster = raster_for(static_cast<long long>(n) * k * sizeof(TIn), false);
-  if (big && opt(kOptRaster) < 0) raster = 8;
+  // Bands of 16 tile rows otherwise: the z-curve's coordinates cost every role up to 1 us of divisions before its first tile
+  // (8943 x 1591 x 506 NT half 27.1 -> 25.5, 1800 x 2448 x 260 NT 14.5 -> 13.4, 901 x 3318 x 275 and single tiles level).
+  const int raster = opt(kOptRaster) >= 0 ? opt(kOptRaster) : (big ? 8 : 16);
   // With the bands, the band's panel of A is what later waves read again and B streams past once per band:
   // A is loaded evict-last, B evict-first.  Same shape: DRAM reads 26.2 -> 17.6 GB per launch, 23.9 -> 22.4 ms.
   unsigned long long hint_a = big ? kL2EvictLast : kL2EvictNormal, hint_b = big ? kL2EvictFirst : kL2EvictNormal;
@@ -671,7 +720,7 @@ int launch_oft_gt(int m, int n, int k, int group_size, const void* A, int ldA, c
   // The options raster, tile_sync and l2_hints override each of them.
   const long long operand_bytes = (static_cast<long long>(m) + n) * k * 2;
   const bool big = kOftPair && operand_bytes > 3ll * st->l2_bytes / 2;
-  const int raster = raster_for(operand_bytes, true);
+  const int raster = opt(kOptRaster) >= 0 ? opt(kOptRaster) : (operand_bytes > (40ll << 20) ? 8 : 0);
   const bool streams = big && static_cast<long long>(n) * k * 2 > st->l2_bytes;  // B does not fit L2: it streams past the band
   unsigned long long hint_a = streams ? kL2EvictLast : kL2EvictNormal, hint_b = streams ? kL2EvictFirst : kL2EvictNormal;
   if (const int h = opt(kOptL2Hints); h >= 0) { hint_a = hint_word(h / 10); hint_b = hint_word(h % 10); }

@@ -546,6 +546,26 @@ __device__ __forceinline__ void umma_tf32_ss_pair(uint32_t d_tmem, uint64_t a_de
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// Two MMAs with the same A operand, which stays in the collector buffer from the first to the second.
+template <int kFmt>
+__device__ __forceinline__ void umma_ss_pair_keep_a(uint32_t d0, uint32_t d1, uint64_t a_desc, uint64_t b0_desc, uint64_t b1_desc, uint32_t idesc,
+                                                    uint32_t accumulate) {
+  if constexpr (kFmt == 0) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %6, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16.collector::a::fill [%0], %2, %3, %5, p;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16.collector::a::lastuse [%1], %2, %4, %5, p;\n\t}"
+        ::"r"(d0), "r"(d1), "l"(a_desc), "l"(b0_desc), "l"(b1_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+  } else {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %6, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::tf32.collector::a::fill [%0], %2, %3, %5, p;\n\t"
+        "tcgen05.mma.cta_group::2.kind::tf32.collector::a::lastuse [%1], %2, %4, %5, p;\n\t}"
+        ::"r"(d0), "r"(d1), "l"(a_desc), "l"(b0_desc), "l"(b1_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+  }
+}
 __device__ __forceinline__ void umma_f16_ts_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
