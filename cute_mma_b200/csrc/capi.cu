@@ -322,19 +322,18 @@ thread_local bool g_whole_k = false;
 // size; plus fixed costs.  What it picks takes 1.2 % longer than the better of the two on average, at worst 14 % (10072 x
 // 181 x 799 NT half 15.2 against 13.4).  5936 x 776 x 5822 NT: 118 against 68 us; 2815 x 6280 x 163: 27 against 20; 11904 x 276 x
 // 263 TF32: 9.9 against 15.7.
-// With K whole (the GEMMs of oft_two_pass, n the rows of X) few rows only, and up to 64 K steps in the first range.  More
-// rows than one tile go either way behind the rotation pass (us on the pair kernel / on this one: 4571 x 4483 x 256 26.7 /
-// 30.0, 852 x 5069 x 2880 41.7 / 27.8); at no more than one tile per SM 96 tiles of 64 steps take 36.9 / 29.6, 128 tiles of
-// 226 steps 85 / 97.9.
+// With K whole (the GEMMs of oft_two_pass, n the rows of X) the model decides in the first range too, where a K step of an SM's only
+// tile costs 0.4 us: 96 tiles of 64 steps 29.6 us against 36.9, 128 tiles of 226 steps 97.9 against 85; 280 tiles of 45
+// steps 27.8 / 41.7, 1296 tiles of 4 steps 30.0 / 26.7.
 bool small_wins(int m, int n, int steps, bool whole_k, const DeviceState* st) {
-  const long long t128 = tiles_128(m, n), pairs = st->sm_count / 2;
-  if (whole_k && (n > 128 || (t128 <= st->sm_count && steps > 64))) return false;
-  if (t128 <= st->sm_count || n <= 128) return true;
+  const long long t128 = tiles_128(m, n), sms = st->sm_count, pairs = sms / 2;
+  if (n <= 128 ? !whole_k || t128 > sms : !whole_k && t128 <= sms) return true;
   const long long t256 = ((static_cast<long long>(m) + 255) / 256) * ((static_cast<long long>(n) + 255) / 256);
-  const long long waves = t128 / (2 * st->sm_count), rest = t128 % (2 * st->sm_count);
+  const long long waves = t128 / (2 * sms), rest = t128 % (2 * sms);
   const int tiles_n = (n + 127) / 128;
   const double step = (n + tiles_n - 1) / tiles_n / 128.0 * steps;  // K steps of 128 columns
-  const double small = 7.0 + step * (0.74 * waves + (rest == 0 ? 0.0 : rest <= st->sm_count ? 0.24 : 0.48)) + 1.2 * (waves + (rest > 0));
+  const double small = t128 <= sms ? 6.0 + 0.4 * step
+                                   : 7.0 + step * (0.74 * waves + (rest == 0 ? 0.0 : rest <= sms ? 0.24 : 0.48)) + 1.2 * (waves + (rest > 0));
   const double pair = 8.0 + static_cast<double>((t256 + pairs - 1) / pairs) * (0.34 * steps + 1.4);
   return small < pair;
 }
@@ -343,11 +342,13 @@ bool small_wins(int m, int n, int steps, bool whole_k, const DeviceState* st) {
 // same number of 256-column tiles, `rounds`; the wide one moves a quarter less between L2 and the SMs and starts with bigger
 // loads, so it needs a second round to pair up and some work to make up for the start.  us on tiles of 256 / 512, 64 random
 // shapes: 12800 x 1123 x 2686 TN 82 / 82, 8192^3 864 / 842, 4690 x 9804 x 9607 NT 906 / 782, TF32 NT 5933 x 7743 x 6727 1331 / 1000;
-// below the lines 1634 x 4191 x 725 TF32 TN (46 K steps in a row) 25 / 26.5, 1296 x 9592 x 349 NT (24) 24.7 / 25.6, above them
-// 3257 x 3051 x 1588 (75) 38.8 / 37.2, NT 12072 x 776 x 421 (21) 23.4 / 21.1, 9304 x 808 x 1265 (40) 29.2 / 27.2.
+// below the lines 1634 x 4191 x 725 TF32 TN (46 K steps in a row) 25 / 26.5, 3658 x 3972 x 551 NT half (36) 25.3 / 26.9, above
+// them 3257 x 3051 x 1588 NT half (75) 38.8 / 37.2, 9304 x 808 x 1265 NT (40) 29.2 / 27.2.  Short tiles of TN products are bound by
+// their stores, which come in bursts here: 13171 x 10088 x 256 125 / 138, 8192 x 8192 x 512 69 / 72, 12667 x 14415 x 701 277 / 256.
+// Not faster, and left: TN of K around 4800 with few rounds (3280 x 6796 x 4735 171 / 175, 1877 x 4397 x 4896 74 / 75).
 bool wide_wins(int m, int n, int steps, bool nt, const DeviceState* st) {
   const long long pairs = st->sm_count / 2, tiles = static_cast<long long>((m + 255) / 256) * ((n + 255) / 256), rounds = (tiles + pairs - 1) / pairs;
-  return n > 256 && rounds >= 2 && rounds * steps >= (nt ? 40 : 60);
+  return n > 256 && rounds >= 2 && rounds * steps >= (nt ? 40 : 60) && (nt || steps > 8);
 }
 
 // What the geometry of a launch depends on beside the sizes: an instance of small_kernel.
@@ -707,8 +708,8 @@ int launch_oft_gt(int m, int n, int k, int group_size, const void* A, int ldA, c
   if (int rc = make_map(&mb, B, 2, k, n, ldB, T::kBK, T::kBN / kRowsPerCta / kGT, "B")) return rc;  // one copy per N-group of the tile
   // Tile order, L2 eviction priorities and the cross-CTA phase lock (pair kernel), chosen by the size of the two
   // operands together, (M + N) K fp16:
-  //  * above 40 MB: bands of 8 tile rows instead of the z-curve (unthrottled launches under ncu, projection shape
-  //    M 16384, K = N 4096, b 64: 438 -> 427 us, DRAM reads 372 -> 344 MB);
+  //  * bands of 8 tile rows: projection shape M 16384, K = N 4096, b 64 438 -> 427 us against the z-curve (unthrottled
+  //    launches under ncu), DRAM reads 372 -> 344 MB; small shapes save its divisions, 16245 x 512 x 320 b 64 16.9 -> 14.6 us;
   //  * above 1.5 x L2 also the phase lock (without it the CTAs drift apart by up to a tile time, the panels that
   //    concurrently running tiles share fall out of L2 before the second reader arrives, and DRAM traffic grew
   //    to 17x the algorithmic bytes at M 65536, N 28672, K 8192: 650-730 -> 795-820 TFLOP/s with the lock) and
@@ -720,7 +721,7 @@ int launch_oft_gt(int m, int n, int k, int group_size, const void* A, int ldA, c
   // The options raster, tile_sync and l2_hints override each of them.
   const long long operand_bytes = (static_cast<long long>(m) + n) * k * 2;
   const bool big = kOftPair && operand_bytes > 3ll * st->l2_bytes / 2;
-  const int raster = opt(kOptRaster) >= 0 ? opt(kOptRaster) : (operand_bytes > (40ll << 20) ? 8 : 0);
+  const int raster = opt(kOptRaster) >= 0 ? opt(kOptRaster) : 8;
   const bool streams = big && static_cast<long long>(n) * k * 2 > st->l2_bytes;  // B does not fit L2: it streams past the band
   unsigned long long hint_a = streams ? kL2EvictLast : kL2EvictNormal, hint_b = streams ? kL2EvictFirst : kL2EvictNormal;
   if (const int h = opt(kOptL2Hints); h >= 0) { hint_a = hint_word(h / 10); hint_b = hint_word(h % 10); }
@@ -789,6 +790,7 @@ constexpr int kNoScratch = -1000;  // internal: no device memory for X.R
 // kOwnScratch bytes of rows at a time and the GEMM's K range is never cut, so that the bits are those of the routes
 // it stands in for.  Not for K above 524288, where that scratch does not hold a row block of 256 rows.
 constexpr size_t kOwnScratch = size_t(256) << 20;
+constexpr size_t kRingBudget = size_t(64) << 20;  // X.R that stays in L2 beside what streams past it: the most a ring of row blocks takes
 size_t xr_row_bytes(int k) { return ((static_cast<size_t>(k) + 7) & ~static_cast<size_t>(7)) * 2; }
 bool two_pass_fits(int k) { return xr_row_bytes(k) * 256 <= kOwnScratch; }
 long long two_pass_rows(int m, int k, bool own) {  // rows of X.R formed at a time; own: two_pass_fits(k)
@@ -861,15 +863,15 @@ RingPlan ring_plan(int m, int n, int k, const DeviceState* st) {
   RingPlan p;
   p.tiles_x = (m + 255) / 256;
   p.tiles_w = (n + 255) / 256;
-  const long long w_bytes = static_cast<long long>(n) * k * 2, mib = 1ll << 20;
+  const long long w_bytes = static_cast<long long>(n) * k * 2, mib = 1ll << 20, most = static_cast<long long>(kRingBudget);
   const bool w_resident = w_bytes <= 64 * mib;
   p.raster = opt(kOptRaster) > 0 ? opt(kOptRaster) : (w_resident ? 4 : 8);
   p.ldx = (static_cast<long long>(k) + 63) & ~63ll;
   const long long block_bytes = 256 * p.ldx * 2;
-  long long budget = 64 * mib;
+  long long budget = most;
   if (w_resident) {
     budget = st->l2_bytes - w_bytes - 16 * mib;
-    budget = budget < 32 * mib ? 32 * mib : (budget > 64 * mib ? 64 * mib : budget);
+    budget = budget < most / 2 ? most / 2 : (budget > most ? most : budget);
   }
   p.bands = static_cast<int>(budget / (block_bytes * p.raster));
   if (p.bands < 2) p.bands = 2;
@@ -1063,7 +1065,8 @@ bool oft_takes_small(const Whole& w, int m, int n, int group_size, int k, int b,
 bool wide_group(int group_size, int b) { return group_size >= (b >= 128 ? 4 : 8) * static_cast<int>(CurrCompParams::bN); }
 
 // aligned: rows of C start on 16-byte boundaries.  *pieces: those of K on route 5.
-int choose_route(int m, int n, int group_size, int k, int b, bool aligned, const DeviceState* st, int* pieces) {
+// two_passes: they are to be had (there is memory for X.R).
+int choose_route(int m, int n, int group_size, int k, int b, bool aligned, const DeviceState* st, int* pieces, bool two_passes = true) {
   int path = g_oft_path != 0 ? g_oft_path : opt(kOptOftRoute);
   const bool can_share = kOftPair && st->pool != nullptr;  // routes 2, 3 and 4 need scratch from the pool
   const Whole w = g_whole.m > 0 ? g_whole : Whole{m, n, group_size};
@@ -1082,10 +1085,19 @@ int choose_route(int m, int n, int group_size, int k, int b, bool aligned, const
   // serialise the rotation with (647 x 4096 x 512 b 64 14.8 / 21.2 / 21.8).  Few rows of X: the GEMM runs on small_kernel, 1 x
   // 131072 x 448 b 64 38 / 29 / 44.
   const bool group_ok = group_size == n || group_size % static_cast<int>(CurrCompParams::bN) == 0;  // what the fused routes take of these widths
-  if (g_more.n == 0 && group_ok && two_pass_fits(k)) {
+  if (two_passes && g_more.n == 0 && group_ok && two_pass_fits(k)) {
     if (!aligned && group_size == n) return 2;
     const long long t256 = ((static_cast<long long>(m) + 255) / 256) * ((static_cast<long long>(group_size) + 255) / 256);
     if (wide && k_steps < 16 && t256 > st->sm_count / 2) return 2;
+    // X.R that stays in L2 between the passes (at most what the ring would hold), and enough N tiles to pay for it: the wide GEMM
+    // behind it has two accumulators and moves less, and neither launch waits for the SMs to be free together.  us on the
+    // best of routes 1, 3, 4 / two passes: 3001 x 11008 x 4096 b 32 247 / 233, 2052 x 13312 x 3296 b 32 171 / 160, 1640 x 3712 x 5696 b 64
+    // 86 / 76, 4820 x 1984 x 1088 b 64 32 / 28, 184 x 17024 x 2176 b 64 25 / 23, 222 x 13248 x 3328 b 128 36 / 30.  Few N tiles pay only
+    // where K is short, the fused kernel's hand-off shows there: 36318 x 640 x 320 b 32 39 / 33, but 9599 x 896 x 2304 b 64 56 / 61.
+    // One round of tiles or 128 x 128 blocks only with few rows (level or not measured above).
+    if (xr_row_bytes(k) * m < kRingBudget && group_size > (k_steps <= 8 ? 2 : 4) * static_cast<int>(CurrCompParams::bN) &&
+        (m < 1024 || (b < 128 && t256 > st->sm_count / 2)))
+      return 2;
   }
   if (!wide) return 1;
   if (g_more.n > 0) return 3;  // of the ring kernels, only oft3_kernel stores to further destinations
@@ -1111,7 +1123,8 @@ int launch_oft(int m, int n, int k, int group_size, const void* A, int ldA, cons
                void* C, int ldC, cudaStream_t stream, DeviceState* st) {
   constexpr int kBN = CurrCompParams::bN;
   int pieces = 1;
-  const int route = choose_route(m, n, group_size, k, kB, (reinterpret_cast<uintptr_t>(C) & 15) == 0 && (ldC & 7) == 0, st, &pieces);
+  const bool aligned = (reinterpret_cast<uintptr_t>(C) & 15) == 0 && (ldC & 7) == 0;
+  int route = choose_route(m, n, group_size, k, kB, aligned, st, &pieces);
   const bool own = g_oft_path != 2 && opt(kOptOftRoute) != 2;
   // A captured call allocates nodes of its graph, which then can be no child graph or conditional body: narrow groups,
   // which no other route needs scratch for, stay off the two passes there.
@@ -1119,7 +1132,8 @@ int launch_oft(int m, int n, int k, int group_size, const void* A, int ldA, cons
     const int rc = oft_two_pass<kB>(m, n, k, group_size, A, ldA, B, ldB, R, ldR, C, ldC, stream, st, own);
     if (rc != kNoScratch) return rc;
     if (g_oft_path == 2) return fail(B200_ECUDA, "no device memory for the %lld bytes of X.R scratch", static_cast<long long>(m) * ((k + 7) & ~7) * 2);
-    // out of memory for X.R: the kernel that keeps X.R in tensor memory needs no scratch
+    // out of memory for X.R: a ring needs less, the kernel that keeps X.R in tensor memory none
+    if (own && aligned) route = choose_route(m, n, group_size, k, kB, aligned, st, &pieces, false);
   }
   if constexpr (kOftPair) {
     if (route == 5 && small_group_ok(n, group_size, kB)) {
