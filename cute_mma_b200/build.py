@@ -13,6 +13,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
@@ -45,8 +46,26 @@ def _stale(out: str, config_dir: str) -> bool:
     return any(os.path.getmtime(d) > t for d in deps if os.path.exists(d))
 
 
+BINDING_SRC = os.path.join(PKG, "binding", "call.c")
+BINDING_OUT = os.path.join(PKG, "_call.so")
+
+
+def build_binding(force: bool = False) -> str:
+    """The CPython module that ops.py calls the C ABI through (plain C, no CUDA)."""
+    if not force and os.path.exists(BINDING_OUT) and os.path.getmtime(BINDING_OUT) >= os.path.getmtime(BINDING_SRC):
+        return BINDING_OUT
+    cmd = [shutil.which("gcc") or "gcc", "-O2", "-Wall", "-shared", "-fPIC", f"-I{sysconfig.get_paths()['include']}", BINDING_SRC, "-o", BINDING_OUT]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        sys.stderr.write(res.stdout + res.stderr)
+        raise RuntimeError("gcc failed: " + " ".join(cmd))
+    return BINDING_OUT
+
+
 def build(config_dir: str = DEFAULT_CONFIG, out: str = DEFAULT_OUT, verbose: bool = False, force: bool = False,
           defines: list[str] | None = None) -> str:
+    if out == DEFAULT_OUT:
+        build_binding(force)
     if not force and not _stale(out, config_dir):
         return out
     cmd = [nvcc_path(), *NVCC_FLAGS, f"-I{config_dir}", f"-I{CSRC}", *(defines or [])]

@@ -16,6 +16,11 @@ import ctypes
 import json
 import os
 
+try:
+    from . import _call  # binding/call.c
+except ImportError:  # not built (build.py makes it): calls go through ctypes
+    _call = None
+
 _PKG = os.path.dirname(os.path.abspath(__file__))
 _LIB_ENV = "CUTE_MMA_B200_LIB"
 
@@ -87,9 +92,23 @@ def load_library(path: str | None = None):
     for name in SYMBOLS:
         if name not in ("b200_kernel_info", "b200_last_error"):
             getattr(lib, name).restype = ctypes.c_int
+    for name, kind in _DIRECT.items():
+        fn = getattr(lib, name)
+        setattr(lib, "direct_" + name, _call.bind(kind, ctypes.cast(fn, vp).value) if _call is not None else _not_taken)
     if path is None:
         _lib = lib
     return lib
+
+
+# Entry points that are called per layer: direct_<name> of a loaded library is a callable of the _call module (binding/call.c),
+# which costs a third of a call through ctypes.  It returns None, having done nothing, for arguments it does not know; the
+# functions below then go through ctypes.
+_DIRECT = {"b200_oft_tn_f16": "oft", "b200_oft_tn_f16_two_pass": "oft", "b200_oft_tn_f16_a_rw": "oft", "b200_gemm_tn_f16": "gemm", "b200_gemm_nt_f16": "gemm",
+           "b200_gemm_tn_tf32": "gemm", "b200_gemm_nt_tf32": "gemm", "b200_gemm_ex": "ex"}
+
+
+def _not_taken(*args):
+    return None
 
 
 def _ptr(x) -> int:
@@ -120,7 +139,11 @@ def oft_tn(m, n, k, A, ldA, B, ldB, R, ldR, C, ldC, stream=None, *, group_size=N
     group_size defaults to n (one block-diagonal R for all of N)."""
     lib = lib or load_library()
     gs = n if group_size is None else group_size
-    _check(lib, lib.b200_oft_tn_f16(m, n, k, gs, reconn_sz, _ptr(A), ldA, _ptr(B), ldB, _ptr(R), ldR, _ptr(C), ldC, _stream(stream)))
+    rc = lib.direct_b200_oft_tn_f16(m, n, k, gs, reconn_sz, A, ldA, B, ldB, R, ldR, C, ldC, stream)
+    if rc is None:
+        rc = lib.b200_oft_tn_f16(m, n, k, gs, reconn_sz, _ptr(A), ldA, _ptr(B), ldB, _ptr(R), ldR, _ptr(C), ldC, _stream(stream))
+    if rc != OK:
+        _check(lib, rc)
 
 
 def oft_tn_two_pass(m, n, k, A, ldA, B, ldB, R, ldR, C, ldC, stream=None, *, group_size=None, reconn_sz=8, lib=None) -> None:
@@ -129,7 +152,11 @@ def oft_tn_two_pass(m, n, k, A, ldA, B, ldB, R, ldR, C, ldC, stream=None, *, gro
     header)."""
     lib = lib or load_library()
     gs = n if group_size is None else group_size
-    _check(lib, lib.b200_oft_tn_f16_two_pass(m, n, k, gs, reconn_sz, _ptr(A), ldA, _ptr(B), ldB, _ptr(R), ldR, _ptr(C), ldC, _stream(stream)))
+    rc = lib.direct_b200_oft_tn_f16_two_pass(m, n, k, gs, reconn_sz, A, ldA, B, ldB, R, ldR, C, ldC, stream)
+    if rc is None:
+        rc = lib.b200_oft_tn_f16_two_pass(m, n, k, gs, reconn_sz, _ptr(A), ldA, _ptr(B), ldB, _ptr(R), ldR, _ptr(C), ldC, _stream(stream))
+    if rc != OK:
+        _check(lib, rc)
 
 
 def rotate(m, k, A, ldA, R, ldR, XR, ldX, stream=None, *, reconn_sz=8, lib=None) -> None:
@@ -254,7 +281,11 @@ def oft_tn_a_rw(m, n, k, A, ldA, B, ldB, R, ldR, C, ldC, stream=None, *, group_s
     """Same product as oft_tn computed as X . (R . W): weight transform, then one plain GEMM."""
     lib = lib or load_library()
     gs = n if group_size is None else group_size
-    _check(lib, lib.b200_oft_tn_f16_a_rw(m, n, k, gs, reconn_sz, _ptr(A), ldA, _ptr(B), ldB, _ptr(R), ldR, _ptr(C), ldC, _stream(stream)))
+    rc = lib.direct_b200_oft_tn_f16_a_rw(m, n, k, gs, reconn_sz, A, ldA, B, ldB, R, ldR, C, ldC, stream)
+    if rc is None:
+        rc = lib.b200_oft_tn_f16_a_rw(m, n, k, gs, reconn_sz, _ptr(A), ldA, _ptr(B), ldB, _ptr(R), ldR, _ptr(C), ldC, _stream(stream))
+    if rc != OK:
+        _check(lib, rc)
 
 
 def oft_tn_host(m, n, k, A, ldA, B, ldB, R, ldR, C, ldC, *, group_size=None, reconn_sz=8, lib=None) -> None:
@@ -264,19 +295,24 @@ def oft_tn_host(m, n, k, A, ldA, B, ldB, R, ldR, C, ldC, *, group_size=None, rec
     _check(lib, lib.b200_oft_tn_f16_host(m, n, k, gs, reconn_sz, _ptr(A), ldA, _ptr(B), ldB, _ptr(R), ldR, _ptr(C), ldC))
 
 
-def _gemm(fn_name, m, n, k, A, ldA, B, ldB, C, ldC, stream, lib):
-    lib = lib or load_library()
-    _check(lib, getattr(lib, fn_name)(m, n, k, _ptr(A), ldA, _ptr(B), ldB, _ptr(C), ldC, _stream(stream)))
-
-
 def gemm_tn(m, n, k, A, ldA, B, ldB, C, ldC, stream=None, *, dtype="half", lib=None) -> None:
     """C(i,j) = sum_l A[i*ldA+l] B[j*ldB+l], C column-major.  dtype 'half' or 'float' (TF32)."""
-    _gemm("b200_gemm_tn_f16" if dtype == "half" else "b200_gemm_tn_tf32", m, n, k, A, ldA, B, ldB, C, ldC, stream, lib)
+    lib = lib or load_library()
+    rc = (lib.direct_b200_gemm_tn_f16 if dtype == "half" else lib.direct_b200_gemm_tn_tf32)(m, n, k, A, ldA, B, ldB, C, ldC, stream)
+    if rc is None:
+        rc = (lib.b200_gemm_tn_f16 if dtype == "half" else lib.b200_gemm_tn_tf32)(m, n, k, _ptr(A), ldA, _ptr(B), ldB, _ptr(C), ldC, _stream(stream))
+    if rc != OK:
+        _check(lib, rc)
 
 
 def gemm_nt(m, n, k, A, ldA, B, ldB, C, ldC, stream=None, *, dtype="half", lib=None) -> None:
     """C(i,j) = sum_l A[i+l*ldA] B[j+l*ldB], C column-major."""
-    _gemm("b200_gemm_nt_f16" if dtype == "half" else "b200_gemm_nt_tf32", m, n, k, A, ldA, B, ldB, C, ldC, stream, lib)
+    lib = lib or load_library()
+    rc = (lib.direct_b200_gemm_nt_f16 if dtype == "half" else lib.direct_b200_gemm_nt_tf32)(m, n, k, A, ldA, B, ldB, C, ldC, stream)
+    if rc is None:
+        rc = (lib.b200_gemm_nt_f16 if dtype == "half" else lib.b200_gemm_nt_tf32)(m, n, k, _ptr(A), ldA, _ptr(B), ldB, _ptr(C), ldC, _stream(stream))
+    if rc != OK:
+        _check(lib, rc)
 
 
 def gemm(transA, transB, m, n, k, A, ldA, B, ldB, C, ldC, stream=None, *, dtype="half", lib=None) -> None:
@@ -291,8 +327,13 @@ F16, F32, TF32 = 0, 1, 2
 def gemm_ex(transA, transB, m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, stream=None, *, in_type=F16, out_type=F16, lib=None) -> None:
     """C (column-major) = alpha * A.B^T + beta * C, half or float result from half operands, float from float (TF32)."""
     lib = lib or load_library()
-    _check(lib, lib.b200_gemm_ex(transA.encode(), transB.encode(), in_type, out_type, m, n, k, float(alpha), _ptr(A), ldA, _ptr(B), ldB,
-                                 float(beta), _ptr(C), ldC, _stream(stream)))
+    alpha, beta = float(alpha), float(beta)
+    rc = lib.direct_b200_gemm_ex(transA, transB, in_type, out_type, m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, stream)
+    if rc is None:
+        rc = lib.b200_gemm_ex(transA.encode(), transB.encode(), in_type, out_type, m, n, k, alpha, _ptr(A), ldA, _ptr(B), ldB, beta, _ptr(C), ldC,
+                              _stream(stream))
+    if rc != OK:
+        _check(lib, rc)
 
 
 def gemm_tn_acc2(m, n, k, A, ldA, B, ldB, k2, A2, ldA2, B2, ldB2, C, ldC, stream=None, *, lib=None) -> None:

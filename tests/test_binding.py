@@ -1,0 +1,60 @@
+"""The compiled binding (binding/call.c) takes what ctypes takes and leaves the rest to it: same status, same exceptions."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from cute_mma_b200 import ops
+
+ADDR = ctypes.addressof((ctypes.c_uint16 * 64)())
+
+
+class Tensor:
+    def __init__(self, at):
+        self.at = at
+
+    def data_ptr(self):
+        return self.at
+
+
+class Stream:
+    cuda_stream = 0
+
+
+# every form of operand and stream the functions document, and sizes that are only int-like
+@pytest.mark.parametrize("x", [ADDR, Tensor(ADDR), np.zeros(64, np.uint16)], ids=["address", "tensor", "array"])
+@pytest.mark.parametrize("stream", [None, 0, Stream()], ids=["none", "address", "stream"])
+@pytest.mark.parametrize("eight", [8, np.int64(8), True + 7], ids=["int", "numpy", "bool"])
+def test_empty_products_are_accepted(lib, x, stream, eight):
+    ops.oft_tn(0, eight, 8, x, 8, x, 8, x, 8, x, 8, stream, reconn_sz=8, lib=lib)
+    ops.gemm_tn(0, eight, 8, x, 8, x, 8, x, 8, stream, lib=lib)
+    ops.gemm_nt(0, eight, 8, x, 8, x, 8, x, 8, stream, dtype="float", lib=lib)
+    ops.gemm_ex("N", "T", 0, eight, 8, 1, x, 8, x, 8, 0, x, 8, stream, out_type=ops.F32, lib=lib)
+
+
+def test_errors_are_those_of_the_ctypes_path(lib, monkeypatch):
+    calls = [lambda: ops.oft_tn(8, 8, 12, ADDR, 16, ADDR, 16, ADDR, 16, ADDR, 8, reconn_sz=8, lib=lib),
+             lambda: ops.oft_tn(8, 8, 16, None, 16, ADDR, 16, ADDR, 16, ADDR, 8, reconn_sz=8, lib=lib),
+             lambda: ops.oft_tn(8, 8, "16", ADDR, 16, ADDR, 16, ADDR, 16, ADDR, 8, reconn_sz=8, lib=lib),
+             lambda: ops.gemm_tn(-1, 8, 8, ADDR, 8, ADDR, 8, ADDR, 8, lib=lib),
+             lambda: ops.gemm_tn(8.0, 8, 8, ADDR, 8, ADDR, 8, ADDR, 8, lib=lib),
+             lambda: ops.gemm_tn(8, 8, 8, "a", 8, ADDR, 8, ADDR, 8, lib=lib),
+             lambda: ops.gemm_tn(8, 8, 8, ADDR, 8, ADDR, 8, ADDR, 8, "stream", lib=lib),
+             lambda: ops.gemm_ex("N", "N", 8, 8, 8, 1.0, ADDR, 8, ADDR, 8, 0.0, ADDR, 8, lib=lib),
+             lambda: ops.gemm_ex("NN", "T", 8, 8, 8, 1.0, ADDR, 8, ADDR, 8, 0.0, ADDR, 8, lib=lib)]
+
+    def seen(call):
+        with pytest.raises(Exception) as e:
+            call()
+        return type(e.value), str(e.value)
+
+    direct = [seen(c) for c in calls]
+    for name in ops._DIRECT:
+        monkeypatch.setattr(lib, "direct_" + name, ops._not_taken)
+    assert direct == [seen(c) for c in calls]
+
+
+def test_the_binding_is_the_path_taken(lib):
+    assert ops._call is not None
+    assert lib.direct_b200_gemm_tn_f16(0, 8, 8, ADDR, 8, ADDR, 8, ADDR, 8, None) == ops.OK
+    assert lib.direct_b200_gemm_tn_f16(0, 8, 8, ADDR, 8, ADDR, 8, ADDR, 8) is None
