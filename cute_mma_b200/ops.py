@@ -148,7 +148,7 @@ def oft_tn(m, n, k, A, ldA, B, ldB, R, ldR, C, ldC, stream=None, *, group_size=N
 
 def oft_tn_two_pass(m, n, k, A, ldA, B, ldB, R, ldR, C, ldC, stream=None, *, group_size=None, reconn_sz=8, lib=None) -> None:
     """oft_tn as a rotation pass (X.R written once to device scratch) followed by the plain GEMM, the route oft_tn takes by
-    itself for short K in wide groups and for one group with unaligned rows of C (see b200_oft_tn_f16_two_pass in the
+    itself for short K in wide groups, for one group with unaligned rows of C and where X.R stays in L2 (see b200_oft_tn_f16_two_pass in the
     header)."""
     lib = lib or load_library()
     gs = n if group_size is None else group_size
