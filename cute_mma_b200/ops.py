@@ -16,11 +16,6 @@ import ctypes
 import json
 import os
 
-try:
-    from . import _call  # binding/call.c
-except ImportError:  # not built (build.py makes it): calls go through ctypes
-    _call = None
-
 _PKG = os.path.dirname(os.path.abspath(__file__))
 _LIB_ENV = "CUTE_MMA_B200_LIB"
 
@@ -92,6 +87,10 @@ def load_library(path: str | None = None):
     for name in SYMBOLS:
         if name not in ("b200_kernel_info", "b200_last_error"):
             getattr(lib, name).restype = ctypes.c_int
+    try:
+        from . import _call  # binding/call.c, built beside the library
+    except ImportError:  # not built: calls go through ctypes
+        _call = None
     for name, kind in _DIRECT.items():
         fn = getattr(lib, name)
         setattr(lib, "direct_" + name, _call.bind(kind, ctypes.cast(fn, vp).value) if _call is not None else _not_taken)
