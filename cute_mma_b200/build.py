@@ -47,36 +47,46 @@ def _stale(out: str, config_dir: str) -> bool:
 
 
 BINDING_SRC = os.path.join(PKG, "binding", "call.c")
-BINDING_OUT = os.path.join(PKG, "_call.so")
+# named for the interpreter it was compiled against: another one neither imports it nor takes it for its own
+BINDING_OUT = os.path.join(PKG, "_call" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 
 
-def build_binding(force: bool = False) -> str:
-    """The CPython module that ops.py calls the C ABI through (plain C, no CUDA)."""
+def build_binding(force: bool = False) -> str | None:
+    """The CPython module that ops.py calls the C ABI through (plain C, no CUDA).  None, with the reason on stderr, where
+    it cannot be built (no compiler, no Python headers): calls then go through ctypes, and the library is none the worse."""
+    untagged = os.path.join(os.path.dirname(BINDING_OUT), "_call.so")
+    if untagged != BINDING_OUT and os.path.exists(untagged):  # any interpreter would import it
+        os.remove(untagged)
     if not force and os.path.exists(BINDING_OUT) and os.path.getmtime(BINDING_OUT) >= os.path.getmtime(BINDING_SRC):
         return BINDING_OUT
     cmd = [shutil.which("gcc") or "gcc", "-O2", "-Wall", "-shared", "-fPIC", f"-I{sysconfig.get_paths()['include']}", BINDING_SRC, "-o", BINDING_OUT]
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-        sys.stderr.write(res.stdout + res.stderr)
-        raise RuntimeError("gcc failed: " + " ".join(cmd))
+    try:
+        res = subprocess.run(cmd, capture_output=True, text=True)
+        failed, why = res.returncode != 0, res.stdout + res.stderr
+    except OSError as e:
+        failed, why = True, f"{e}\n"
+    if failed:
+        if os.path.exists(BINDING_OUT):  # of an older source, which may not fit the library any more
+            os.remove(BINDING_OUT)
+        sys.stderr.write(why + "no compiled binding, calls go through ctypes: " + " ".join(cmd) + "\n")
+        return None
     return BINDING_OUT
 
 
 def build(config_dir: str = DEFAULT_CONFIG, out: str = DEFAULT_OUT, verbose: bool = False, force: bool = False,
           defines: list[str] | None = None) -> str:
+    if force or _stale(out, config_dir):
+        cmd = [nvcc_path(), *NVCC_FLAGS, f"-I{config_dir}", f"-I{CSRC}", *(defines or [])]
+        if verbose:
+            cmd += ["-Xptxas", "-v"]
+        cmd += sources() + ["-o", out, "-lcudart"]
+        res = subprocess.run(cmd, capture_output=True, text=True)
+        if verbose or res.returncode != 0:
+            sys.stderr.write(res.stdout + res.stderr)
+        if res.returncode != 0:
+            raise RuntimeError("nvcc failed: " + " ".join(cmd))
     if out == DEFAULT_OUT:
         build_binding(force)
-    if not force and not _stale(out, config_dir):
-        return out
-    cmd = [nvcc_path(), *NVCC_FLAGS, f"-I{config_dir}", f"-I{CSRC}", *(defines or [])]
-    if verbose:
-        cmd += ["-Xptxas", "-v"]
-    cmd += sources() + ["-o", out, "-lcudart"]
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if verbose or res.returncode != 0:
-        sys.stderr.write(res.stdout + res.stderr)
-    if res.returncode != 0:
-        raise RuntimeError("nvcc failed: " + " ".join(cmd))
     return out
 
 

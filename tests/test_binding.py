@@ -1,10 +1,12 @@
 """The compiled binding (binding/call.c) takes what ctypes takes and leaves the rest to it: same status, same exceptions."""
 import ctypes
+import os
+import sysconfig
 
 import numpy as np
 import pytest
 
-from cute_mma_b200 import ops
+from cute_mma_b200 import build, ops
 
 ADDR = ctypes.addressof((ctypes.c_uint16 * 64)())
 
@@ -55,5 +57,34 @@ def test_errors_are_those_of_the_ctypes_path(lib, monkeypatch):
 
 
 def test_the_binding_is_the_path_taken(lib):
+    pytest.importorskip("cute_mma_b200._call", reason="not built here: ctypes is the path")
     assert lib.direct_b200_gemm_tn_f16(0, 8, 8, ADDR, 8, ADDR, 8, ADDR, 8, None) == ops.OK
     assert lib.direct_b200_gemm_tn_f16(0, 8, 8, ADDR, 8, ADDR, 8, ADDR, 8) is None
+
+
+@pytest.fixture
+def another_place(monkeypatch, tmp_path):
+    """The binding built somewhere else, beside an untagged one of an earlier build."""
+    (tmp_path / "_call.so").write_bytes(b"")
+    monkeypatch.setattr(build, "BINDING_OUT", str(tmp_path / os.path.basename(build.BINDING_OUT)))
+    return tmp_path
+
+
+@pytest.mark.parametrize("missing", ["compiler", "headers"])
+def test_the_library_builds_without_the_binding(lib, monkeypatch, another_place, capfd, missing):
+    if missing == "compiler":
+        monkeypatch.setattr(build.shutil, "which", lambda name: str(another_place / name))
+    else:
+        monkeypatch.setattr(build.sysconfig, "get_paths", lambda: {"include": str(another_place)})
+        monkeypatch.setenv("C_INCLUDE_PATH", "")
+    assert build.build() == build.DEFAULT_OUT
+    assert build.build_binding() is None and not os.path.exists(build.BINDING_OUT)
+    assert "ctypes" in capfd.readouterr().err
+
+
+def test_the_binding_belongs_to_its_interpreter(another_place):
+    suffix = sysconfig.get_config_var("EXT_SUFFIX")
+    assert build.BINDING_OUT.endswith(suffix)
+    if build.build_binding() is None:
+        pytest.skip("no C compiler or Python headers here")
+    assert [f.name for f in another_place.iterdir()] == ["_call" + suffix]
