@@ -62,6 +62,32 @@ def test_the_binding_is_the_path_taken(lib):
     assert lib.direct_b200_gemm_tn_f16(0, 8, 8, ADDR, 8, ADDR, 8, ADDR, 8) is None
 
 
+def test_a_library_of_the_callers_own(lib):
+    """lib= takes whatever has the C functions, not only what load_library returned."""
+
+    class Own:
+        b200_last_error = lib.b200_last_error
+
+        def __init__(self):
+            self.seen = []
+
+        def __getattr__(self, name):
+            if not name.startswith("b200_"):
+                raise AttributeError(name)
+            self.seen.append(name)
+            return getattr(lib, name)
+
+    own = Own()
+    ops.oft_tn(0, 8, 8, ADDR, 8, ADDR, 8, ADDR, 8, ADDR, 8, lib=own)
+    ops.oft_tn_two_pass(0, 8, 8, ADDR, 8, ADDR, 8, ADDR, 8, ADDR, 8, lib=own)
+    ops.oft_tn_a_rw(0, 8, 8, ADDR, 8, ADDR, 8, ADDR, 8, ADDR, 8, lib=own)
+    for dtype in ("half", "float"):
+        ops.gemm_tn(0, 8, 8, ADDR, 8, ADDR, 8, ADDR, 8, dtype=dtype, lib=own)
+        ops.gemm_nt(0, 8, 8, ADDR, 8, ADDR, 8, ADDR, 8, dtype=dtype, lib=own)
+    ops.gemm_ex("N", "T", 0, 8, 8, 1, ADDR, 8, ADDR, 8, 0, ADDR, 8, lib=own)
+    assert sorted(own.seen) == sorted(ops._DIRECT)
+
+
 @pytest.fixture
 def another_place(monkeypatch, tmp_path):
     """The binding built somewhere else, beside an untagged one of an earlier build."""
