@@ -1094,8 +1094,11 @@ int choose_route(int m, int n, int group_size, int k, int b, bool aligned, const
     // best of routes 1, 3, 4 / two passes: 3001 x 11008 x 4096 b 32 247 / 233, 2052 x 13312 x 3296 b 32 171 / 160, 1640 x 3712 x 5696 b 64
     // 86 / 76, 4820 x 1984 x 1088 b 64 32 / 28, 184 x 17024 x 2176 b 64 25 / 23, 222 x 13248 x 3328 b 128 36 / 30.  Few N tiles pay only
     // where K is short, the fused kernel's hand-off shows there: 36318 x 640 x 320 b 32 39 / 33, but 9599 x 896 x 2304 b 64 56 / 61.
-    // One round of tiles or 128 x 128 blocks only with few rows (level or not measured above).
-    if (xr_row_bytes(k) * m < kRingBudget && group_size > (k_steps <= 8 ? 2 : 4) * static_cast<int>(CurrCompParams::bN) &&
+    // One round of tiles or 128 x 128 blocks only with few rows (level or not measured above).  Several groups take two launches
+    // each, one group after the other, and so do the rings (484 x 28672 x 1024 b 32 in 7 groups 158 / 89), but route 1 takes all
+    // groups that are not wide in one launch: 1000 x 3840 x 1280 b 64 in 3 groups 17 / 35, 300 x 28160 x 2048 b 64 in 22 54 / 386,
+    // 4104 x 10752 x 1664 b 32 in 7 144 / 239.
+    if ((group_size == n || wide) && xr_row_bytes(k) * m < kRingBudget && group_size > (k_steps <= 8 ? 2 : 4) * static_cast<int>(CurrCompParams::bN) &&
         (m < 1024 || (b < 128 && t256 > st->sm_count / 2)))
       return 2;
   }
