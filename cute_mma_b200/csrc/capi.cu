@@ -347,7 +347,7 @@ bool small_wins(int m, int n, int steps, bool whole_k, const DeviceState* st) {
 // their stores, which come in bursts here: 13171 x 10088 x 256 125 / 138, 8192 x 8192 x 512 69 / 72, 12667 x 14415 x 701 277 / 256.
 // Not faster, and left: TN of K around 4800 with few rounds (3280 x 6796 x 4735 171 / 175, 1877 x 4397 x 4896 74 / 75).
 bool wide_wins(int m, int n, int steps, bool nt, const DeviceState* st) {
-  const long long pairs = st->sm_count / 2, tiles = static_cast<long long>((m + 255) / 256) * ((n + 255) / 256), rounds = (tiles + pairs - 1) / pairs;
+  const long long pairs = st->sm_count / 2, tiles = ((m + 255ll) / 256) * ((n + 255ll) / 256), rounds = (tiles + pairs - 1) / pairs;
   return n > 256 && rounds >= 2 && rounds * steps >= (nt ? 40 : 60) && (nt || steps > 8);
 }
 
@@ -507,12 +507,10 @@ int launch_wide(int m, int n, int k, const CUtensorMap& ma, const CUtensorMap& m
   int* rounds = nullptr;
   if (tile_sync)
     if (int rc = round_counters(st, stream, &rounds)) return rc;
-  const long long pairs = st->sm_count / 2, tiles_m = (m + 255) / 256, tiles_n = (n + 255) / 256;
-  const unsigned wide = wide_tiles_whole(tiles_m * (tiles_n / 2), tiles_n % 2 ? tiles_m : 0, pairs);
+  const WideGrid geo = wide_grid(m, n, st->sm_count / 2);
   Gemm2WArgs args{m, n, k, C, ldC, st->status, raster, tile_sync, rounds, a3d, b3d, h >= 0 ? hint_word(h / 10) : kL2EvictNormal,
-                  h >= 0 ? hint_word(h % 10) : kL2EvictNormal, wide, alpha, beta};
-  const long long items = tiles_m * tiles_n - wide;
-  const int grid = 2 * static_cast<int>(items < pairs ? items : pairs);
+                  h >= 0 ? hint_word(h % 10) : kL2EvictNormal, geo.wide, alpha, beta};
+  const int grid = 2 * static_cast<int>(geo.pairs);
   cudaError_t e = cudaErrorUnknown;
   if (args.tile_sync && (e = launch_cooperative(kernel, grid, T::kThreads, T::kSmemBytes, stream, ma, mb, args)) != cudaSuccess) {
     cudaGetLastError();

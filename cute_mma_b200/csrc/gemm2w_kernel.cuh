@@ -63,7 +63,7 @@ struct Gemm2WArgs {
   int* rounds;                        // 4 zeroed counters (tile_sync only)
   int a3d, b3d;                       // MN-major operand described by a 3-D map
   unsigned long long hint_a, hint_b;  // L2 eviction priority of the K-major tile loads
-  unsigned wide;                      // this many tiles run whole, the halves of the others are items of their own
+  unsigned wide;                      // this many tiles run whole, the halves of the others are items of their own (wide_grid)
   float alpha, beta;
 };
 
@@ -79,26 +79,26 @@ struct WideItem {
 struct WideSchedule {
   unsigned tiles_m, tiles_w, wide, full_rounds, part, split, halves, pairs;
   int raster, last_n0;
-  __device__ WideSchedule(const Gemm2WArgs& args, unsigned num_pairs) {
-    const unsigned tiles_n = (args.n + 255) / 256;
-    tiles_m = (args.m + 255) / 256;
+  __host__ __device__ WideSchedule(int m, int n, unsigned wide_, int raster_, unsigned num_pairs) {
+    const unsigned tiles_n = (n + 255u) / 256;
+    tiles_m = (m + 255u) / 256;
     tiles_w = tiles_n / 2;
-    wide = args.wide;
+    wide = wide_;
     pairs = num_pairs;
     full_rounds = wide / pairs;
     part = wide % pairs;
     split = 2 * (tiles_m * tiles_w - wide);  // halves that come from cut tiles
     halves = split + (tiles_n & 1 ? tiles_m : 0);
-    raster = args.raster;
+    raster = raster_;
     last_n0 = static_cast<int>(tiles_n - 1) * 256;
   }
-  __device__ WideItem tile(unsigned t) const {
+  __host__ __device__ WideItem tile(unsigned t) const {
     unsigned tm, tw;
     tile_coord_r(raster, tiles_m, tiles_w, t, tm, tw);
     return {tm, static_cast<int>(tw) * 512, 2};
   }
   // item j of pair `pair`; false when there is none any more
-  __device__ bool item(unsigned pair, unsigned j, WideItem& w) const {
+  __host__ __device__ bool item(unsigned pair, unsigned j, WideItem& w) const {
     if (j < full_rounds) {
       w = tile(j * pairs + pair);
       return true;
@@ -137,6 +137,16 @@ inline unsigned wide_tiles_whole(long long tiles, long long single_halves, long 
   if (left <= pairs) return static_cast<unsigned>(tiles - rest);
   if (4 * left <= 5 * pairs && left - pairs < rest) return static_cast<unsigned>(tiles - rest + left - pairs);
   return static_cast<unsigned>(tiles);
+}
+// What a launch for an m x n result on a GPU of `pairs` SM pairs needs: the tiles that run whole and the pairs that get work.
+struct WideGrid {
+  unsigned wide, pairs;
+};
+inline WideGrid wide_grid(int m, int n, long long pairs) {
+  const long long tiles_m = (m + 255ll) / 256, tiles_n = (n + 255ll) / 256;
+  const unsigned wide = wide_tiles_whole(tiles_m * (tiles_n / 2), tiles_n % 2 ? tiles_m : 0, pairs);
+  const long long items = tiles_m * tiles_n - wide;
+  return {wide, static_cast<unsigned>(items < pairs ? items : pairs)};
 }
 
 // MMAs of one K step (128 bytes of K): accumulator d0 over the first B tile, d1 over the second, or both with A kept in the
@@ -292,7 +302,7 @@ gemm2w_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant_
   const int warp = warp_id_uniform(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();  // 0 = leader (issues the MMAs), 1 = peer
   const unsigned pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
-  const WideSchedule sched(args, num_pairs);
+  const WideSchedule sched(args.m, args.n, args.wide, args.raster, num_pairs);
   const int k_steps = (args.k + T::kBK - 1) / T::kBK;
 
   if (threadIdx.x == 0) {
