@@ -234,13 +234,14 @@ __device__ __forceinline__ bool wide_issue_item(int halves, int k_steps, uint32_
 template <typename TOut, class Release>
 __device__ __forceinline__ void wide_store(uint32_t t_row, TOut* c, long long ld, int cols, bool whole, float alpha, float beta, Release release) {
   constexpr int kChunks = 4;
-  if (!whole) {  // straight from tensor memory
+  if (!whole) {  // straight from tensor memory; whole blocks of 32 columns in the fast loop, a tile's last rows and columns hold up
+                 // the accumulator (us 2542 x 3175 x 2752 half 37.8 -> 34.0, 2388 x 2312 x 4032 53.8 -> 49.7, 256-column tiles 34.1 and 48.1)
 #pragma unroll 1
     for (int i = 0; i < kChunks; ++i) {
       uint32_t v[32];
       tmem_ld_x32(t_row + i * 32, v);
       tmem_wait_ld();
-      if (cols > 32 * i) store_columns<TOut>(v, c + 32ll * i * ld, ld, cols - 32 * i, alpha, beta, false);
+      if (cols > 32 * i) store_columns<TOut>(v, c + 32ll * i * ld, ld, cols - 32 * i, alpha, beta, true);
     }
     __syncwarp();
     release();

@@ -129,3 +129,27 @@ def test_phase_lock_on_two_streams(lib, cuda, pair_build, wide):
     torch.cuda.synchronize()
     assert ops.device_status(lib)[0] == 0
     assert torch.equal(C[0], C[1]) and torch.equal(C[0], C[2])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("t_in,t_out", [("half", "half"), ("half", "float"), ("float", "float")])
+def test_ragged_edges_are_stored_as_fast(lib, cuda, pair_build, t_in, t_out):
+    """One row and one column less than whole tiles, in the same C: a warp of the last tiles has 128 columns to store with checks,
+    at 4 instructions a column about 1 us more than without, at 16 more than 4."""
+    import torch
+
+    from test_beta_gpu import us
+
+    if not pair_build:
+        pytest.skip("tiles of 256 x 512 belong to the CTA-pair build")
+    m, n, k = 2304, 2048, 512
+    A, B = (torch.randn((r, k), device=cuda).to(torch.float16 if t_in == "half" else torch.float32) for r in (m, n))
+    C = torch.empty((n, m), device=cuda, dtype=torch.float16 if t_out == "half" else torch.float32)
+
+    def call(rows, cols):
+        ops.gemm_ex("T", "N", rows, cols, k, 1.0, A, k, B, k, 0.0, C, m, in_type=ops.F16 if t_in == "half" else ops.TF32,
+                    out_type=ops.F16 if t_out == "half" else ops.F32, lib=lib)
+
+    with ops.option("gemm_wide", 1, lib), ops.option("small_tiles", 0, lib):
+        whole, ragged = us(lambda: call(m, n)), us(lambda: call(m - 1, n - 1))
+    assert ragged - whole <= 2.5, (whole, ragged)
