@@ -24,6 +24,7 @@
 #include "gemm_kernel.cuh"
 #include "gemm2_kernel.cuh"
 #include "gemm2w_kernel.cuh"
+#include "gemm_choice.hpp"
 #include "oft_kernel.cuh"
 #include "oft2_kernel.cuh"
 #include "xr_kernel.cuh"
@@ -307,50 +308,8 @@ struct PartOf {
   PartOf(int m, int n, int group_size) { g_whole.m = m; g_whole.n = n; g_whole.group_size = group_size; }
   ~PartOf() { g_whole = before; }
 };
-// Tiles of 128 x 128 of an m x n result.
-long long tiles_128(int m, int n) { return ((static_cast<long long>(m) + 127) / 128) * ((static_cast<long long>(n) + 127) / 128); }
-
 // Products whose K range must not be cut (the parts of a two-pass product, see oft_two_pass).
 thread_local bool g_whole_k = false;
-
-// Whether small_kernel takes a plain m x n product of `steps` K steps (128 bytes of a row each).
-// As long as its 128 x 128 tiles do not outnumber the SMs, always (fixed cost per launch 5 us against 7 to 9 us, and 256 x
-// 256 tiles leave most SMs idle: 640 x 1280 x 1024 TF32 29 -> 10 us), and for n <= 128, of which a pair tile covers twice
-// the columns at least (65536 x 120 x 4096 half 100 against 128 us, 131072 x 64 x 512 31 against 40).  Above, the two are
-// compared by a model fitted to 550 random shapes of 149 to 1500 tiles: a K step of two tiles per SM costs 0.74 us for 128
-// columns and 0.6 of that for the 128 rows of P alone (a narrow tile loads and multiplies those all the same), a last wave of one tile
-// per SM 0.24 and of more 0.48; a round of pair tiles 0.34 us per step on 74 pairs, either size; plus fixed costs.  What it
-// picks takes 1 % longer than the better of the two on average, at worst 31 % (23650 x 310 x 1485 NT half to float 50.0 us against
-// 38.1).  Counted by its columns alone a narrow tile lost up to 55 % (7016 x 272 x 2536 half 29.5 against 21.0, 33475 x 147 x 2919 67.8
-// against 47.9).  5936 x 776 x 5822 NT: 118 against 68 us; 2815 x 6280 x 163: 27 against 20; 11904 x 276 x 263 TF32: 9.9 against 15.7.
-// With K whole (the GEMMs of oft_two_pass, n the rows of X) the model decides in the first range too, where a K step of an SM's only
-// tile costs 0.4 us: 96 tiles of 64 steps 29.6 us against 36.9, 128 tiles of 226 steps 97.9 against 85; 280 tiles of 45
-// steps 27.8 / 41.7, 1296 tiles of 4 steps 30.0 / 26.7.
-bool small_wins(int m, int n, int steps, bool whole_k, const DeviceState* st) {
-  const long long t128 = tiles_128(m, n), sms = st->sm_count, pairs = sms / 2;
-  if (n <= 128 ? !whole_k || t128 > sms : !whole_k && t128 <= sms) return true;
-  const long long t256 = ((static_cast<long long>(m) + 255) / 256) * ((static_cast<long long>(n) + 255) / 256);
-  const long long waves = t128 / (2 * sms), rest = t128 % (2 * sms);
-  const int tiles_n = (n + 127) / 128;
-  const double step = (0.6 + 0.4 * ((n + tiles_n - 1) / tiles_n) / 128.0) * steps;  // K steps of 128 columns
-  const double small = t128 <= sms ? 6.0 + 0.4 * step
-                                   : 6.0 + step * (0.74 * waves + (rest == 0 ? 0.0 : rest <= sms ? 0.24 : 0.48)) + 1.4 * (waves + (rest > 0));
-  const double pair = 8.0 + static_cast<double>((t256 + pairs - 1) / pairs) * (0.34 * steps + 1.4);
-  return small < pair;
-}
-
-// Whether the plain GEMM of `steps` K steps runs on tiles of 256 x 512 (gemm2w_kernel).  Both kernels give the longest pair the
-// same number of 256-column tiles, `rounds`; the wide one moves a quarter less between L2 and the SMs and starts with bigger
-// loads, so it needs a second round to pair up and some work to make up for the start.  us on tiles of 256 / 512, 64 random
-// shapes: 12800 x 1123 x 2686 TN 82 / 82, 8192^3 864 / 842, 4690 x 9804 x 9607 NT 906 / 782, TF32 NT 5933 x 7743 x 6727 1331 / 1000;
-// below the lines 1634 x 4191 x 725 TF32 TN (46 K steps in a row) 25 / 26.5, 3658 x 3972 x 551 NT half (36) 25.3 / 26.9, above
-// them 3257 x 3051 x 1588 NT half (75) 38.8 / 37.2, 9304 x 808 x 1265 NT (40) 29.2 / 27.2.  Short tiles of TN products are bound by
-// their stores, which come in bursts here: 13171 x 10088 x 256 125 / 138, 8192 x 8192 x 512 69 / 72, 12667 x 14415 x 701 277 / 256.
-// Not faster, and left: TN of K around 4800 with few rounds (3280 x 6796 x 4735 171 / 175, 1877 x 4397 x 4896 74 / 75).
-bool wide_wins(int m, int n, int steps, bool nt, const DeviceState* st) {
-  const long long pairs = st->sm_count / 2, tiles = ((m + 255ll) / 256) * ((n + 255ll) / 256), rounds = (tiles + pairs - 1) / pairs;
-  return n > 256 && rounds >= 2 && rounds * steps >= (nt ? 40 : 60) && (nt || steps > 8);
-}
 
 // What the geometry of a launch depends on beside the sizes: an instance of small_kernel.
 struct SmallKind {
@@ -546,7 +505,7 @@ int launch_gemm_bn(int m, int n, int k, const void* A, int ldA, const void* B, i
   DeviceState* st;
   if (int rc = device_state(&st)) return rc;
   if constexpr (kPair) {
-    if (k2 == 0 && (opt(kOptSmallTiles) < 0 ? small_wins(m, n, (k + T1::kBK - 1) / T1::kBK, g_whole_k, st) : opt(kOptSmallTiles) != 0)) {
+    if (k2 == 0 && (opt(kOptSmallTiles) < 0 ? small_wins(m, n, (k + T1::kBK - 1) / T1::kBK, g_whole_k, st->sm_count) : opt(kOptSmallTiles) != 0)) {
       using TS = SmallTraits<TIn, TOut, kNT, 0>;
       const SmallPlan p = small_plan(small_kind<TS>(), n, k, st);
       return launch_small<TS>(p, g_whole_k ? 1 : small_pieces(small_kind<TS>(), p, m, n), m, n, k, A, ldA, "A", B, ldB, "B", nullptr, 0, 1, C, ldC, alpha, beta, stream, st);
@@ -576,7 +535,8 @@ int launch_gemm_bn(int m, int n, int k, const void* A, int ldA, const void* B, i
   if constexpr (kPair && kBN == 256) {
     using TW = Gemm2WTraits<TIn, TOut, kNT>;
     const int steps = (k + TW::kBK - 1) / TW::kBK;
-    if (k2 == 0 && steps >= TW::kMinSteps && (opt(kOptGemmWide) < 0 ? wide_wins(m, n, steps, kNT, st) : opt(kOptGemmWide) != 0))
+    const bool whole_lines = ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | ldA * sizeof(TIn) | ldB * sizeof(TIn)) & 127) == 0;
+    if (k2 == 0 && steps >= TW::kMinSteps && (opt(kOptGemmWide) < 0 ? wide_wins(m, n, steps, kNT, whole_lines, st->sm_count) : opt(kOptGemmWide) != 0))
       return launch_wide<TW>(m, n, k, ma, mb, a3d, b3d, C, ldC, alpha, beta, operand_bytes, stream, st);
   }
   const bool big = kPair && operand_bytes > 3ll * st->l2_bytes / 2;
