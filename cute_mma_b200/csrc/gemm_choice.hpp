@@ -39,7 +39,7 @@ inline bool small_wins(int m, int n, int steps, bool whole_k, long long sms) {
 // 864 / 842, 4690 x 9804 x 9607 NT 906 / 782, TF32 NT 5933 x 7743 x 6727 1331 / 1000; below the lines 1634 x 4191 x 725 TF32 TN (46 K
 // steps in a row) 25 / 26.5, 3658 x 3972 x 551 NT half (36) 25.3 / 26.9, above them 3257 x 3051 x 1588 NT half (75) 38.8 / 37.2,
 // 9304 x 808 x 1265 NT (40) 29.2 / 27.2.  Short tiles of TN products are bound by their stores, which come in bursts here:
-// 13171 x 10088 x 256 125 / 138, 8192 x 8192 x 512 69 / 72.
+// 13171 x 10088 x 256 98 / 138, 8192 x 8192 x 512 69 / 72.
 // How much the quarter is worth depends on whether the operands' rows start on 128-byte lines (whole_lines).  Where they do not,
 // every 128-byte piece of a tile touches two, and the wide tile takes 0.91 of the other's time on average (190 random shapes above
 // the lines).  Where they do, NT products are level in short runs and 2 % faster in long ones, under the power cap; TN
