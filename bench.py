@@ -548,7 +548,7 @@ def run_gpu_arm(args, workload):
         achieved = flops_launch / (ms * 1e-3) * 1e-12
         timed_s = ms * args.steps * 1e-3
         peak = peaks["bf16_sustained"] if timed_s >= 2.0 else peaks["bf16_burst"]
-        kernel_of = {"fused_ring": "oft3_kernel", "fused_ring_split": "oft4_kernel", "fused_tmem": "oft2_kernel", "two_pass": "xr_kernel + gemm2w_kernel",
+        kernel_of = {"fused_ring": "oft3_kernel", "fused_ring_split": "oft4_kernel", "fused_tmem": "oft2_kernel", "two_pass": "xr_kernel + plain GEMM (gemm2w_kernel, gemm2_kernel or small_kernel by size)",
                      "fused_small": "small_kernel"}
         config_of_route = {"fused_ring": "oft_ring", "fused_ring_split": "oft_ring_split"}
         roofline = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,

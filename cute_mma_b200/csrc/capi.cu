@@ -71,7 +71,7 @@ constexpr OptionDef kOptionDefs[kOptCount] = {
     {"small_split", "B200_SMALL_SPLIT", -1},      // small-problem kernel: pieces along K (1..8)
     {"pdl", "B200_PDL", -1},                      // 0: no programmatic dependent launch
     {"small_stages", "B200_SMALL_STAGES", -1},    // small-problem kernel: ring depth
-    {"gemm_wide", "B200_GEMM_WIDE", -1},          // plain GEMM: 0 never tiles of 256 x 512, 1 always
+    {"gemm_wide", "B200_GEMM_WIDE", -1},          // plain GEMM: 0 never tiles of 256 x 512, 1 wherever pair tiles of 256 x 256 would run and K has 4 steps
 };
 std::atomic<int> g_opt[kOptCount];
 std::once_flag g_opt_once;
@@ -530,7 +530,8 @@ int launch_gemm_bn(int m, int n, int k, const void* A, int ldA, const void* B, i
   // bands of 8 tile rows, 25.7 ms with both (before the L2 eviction priorities below were added).
   // The same three measures already pay when the two operands together exceed one and a half times L2 (one-pass
   // ncu counters, unthrottled launches): 8192^3 fp16 721 -> 689 us and 1.37 -> 0.85 GB of DRAM reads; M 8192,
-  // N 4096, K 8192 354 -> 346 us; 4096 x 16384 x 4096 and below: no difference, so they stay on the z-curve.
+  // N 4096, K 8192 354 -> 346 us; 4096 x 16384 x 4096 and below: no difference, so they go without the lock and the priorities
+  // (their tile order is below).  Products on tiles of 256 x 512 have rules of their own (launch_wide).
   const long long operand_bytes = (static_cast<long long>(m) + n) * k * static_cast<long long>(sizeof(TIn));
   if constexpr (kPair && kBN == 256) {
     using TW = Gemm2WTraits<TIn, TOut, kNT>;
@@ -1057,7 +1058,10 @@ int choose_route(int m, int n, int group_size, int k, int b, bool aligned, const
     // best of routes 1, 3, 4 / two passes: 3001 x 11008 x 4096 b 32 247 / 233, 2052 x 13312 x 3296 b 32 171 / 160, 1640 x 3712 x 5696 b 64
     // 86 / 76, 4820 x 1984 x 1088 b 64 32 / 28, 184 x 17024 x 2176 b 64 25 / 23, 222 x 13248 x 3328 b 128 36 / 30.  Few N tiles pay only
     // where K is short, the fused kernel's hand-off shows there: 36318 x 640 x 320 b 32 39 / 33, but 9599 x 896 x 2304 b 64 56 / 61.
-    // One round of tiles or 128 x 128 blocks only with few rows (level or not measured above).  Several groups take two launches
+    // One round of tiles only with few rows (level above).  The 64 MB, and the 1024 rows from which 128 x 128 blocks stay on the
+    // ring, are not where the two forms cross: two passes are ahead beyond them as well (ring / two passes 32768 x 28672 x 1024 b 64
+    // 2.59 / 1.47 ms, 16384 x 2048 x 4096 b 128 289 / 260 us; 16384 x 4096 x 4096 b 64 492 / 454 in long runs, 480 / 507 in short ones).
+    // They are what b200_oft_plan documents, tests/test_oft_gpu.py pins and callers size their memory by (64 MB of scratch).  Several groups take two launches
     // each, one group after the other, and so do the rings (484 x 28672 x 1024 b 32 in 7 groups 158 / 89), but route 1 takes all
     // groups that are not wide in one launch: 1000 x 3840 x 1280 b 64 in 3 groups 17 / 35, 300 x 28160 x 2048 b 64 in 22 54 / 386,
     // 4104 x 10752 x 1664 b 32 in 7 144 / 239.

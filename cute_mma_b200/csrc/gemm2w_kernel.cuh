@@ -4,11 +4,11 @@
 // Bound: the 1 kW power cap.  The pair kernels reach it whenever launches follow one another for more than some tens of
 // milliseconds, and from there on the energy of a launch is its time (970 to 990 W on every large product, whatever the clock;
 // 8192^3 half on gemm2_kernel 880 mJ, of which moving the operands without a single MMA takes about a third).  A 256 x 256
-// tile loads 32 KB per CTA and 64 columns of K, 9.5 TB/s from L2 at 8192^3; two accumulators of 256 columns that share the rows
+// tile loads 32 KB per CTA and 64 columns of K, 9.9 TB/s from L2 at 8192^3; two accumulators of 256 columns that share the rows
 // of A load 48 KB for twice the work (8.6 -> 6.4 GB in all), and the A operand of a pair of MMAs is fetched from shared memory
 // once (collector buffer, 1 %).  Long runs, us on tiles of 256 / 512: 8192^3 half 864 / 831, 4096 x 4096 x 16384 half NT 471 /
 // 436, 4096^3 TF32 NT 221 / 209, 11008 x 3001 x 4096 half 252 / 219, 16384 x 4096 x 1024 half 130 / 119.  Per 64 columns of K and
-// tile the pipe needs 1024 cycles and the issuer's middle steps take 1004 to 1019; 2300 cycles a tile go into its two ends.
+// tile the pipe needs 1024 cycles, which the middle steps keep to; 2300 cycles a tile go into its two ends.
 //
 // Tensor memory (512 columns) holds the two accumulators of ONE tile, so nothing is left for the next one.  The halves are
 // therefore run kSkew K steps apart at both ends of a tile: at the end, half 0 finishes its last kSkew steps first and its

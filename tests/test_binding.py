@@ -113,3 +113,12 @@ def test_the_binding_belongs_to_its_interpreter(another_place):
     if build.build_binding() is None:
         pytest.skip("no C compiler or Python headers here")
     assert [f.name for f in another_place.iterdir()] == ["_call" + suffix]
+
+
+def test_a_bool_is_an_integer(lib):
+    """As for ctypes: True is a dimension or a leading dimension of 1."""
+    own = type("Own", (), {"b200_last_error": lib.b200_last_error, "b200_gemm_tn_f16": lib.b200_gemm_tn_f16})()
+    for through in (lib, own):  # the binding, ctypes
+        ops.gemm_tn(False, True, 8, ADDR, 8, ADDR, 8, ADDR, True, lib=through)
+        with pytest.raises(ops.Error):
+            ops.gemm_tn(8, True, 8, ADDR, True, ADDR, 8, ADDR, 8, lib=through)

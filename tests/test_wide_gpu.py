@@ -9,8 +9,8 @@ from cute_mma_b200 import ops  # noqa: E402
 pytestmark = pytest.mark.gpu
 
 # (m, n, k): least K of the kernel (4 steps of 64 halves), two halves of one tile, a last half of one column, odd numbers of 256-column
-# tiles (whole tiles beside single halves), whole rounds of 74 pairs with halves behind them, and a part-filled round of whole
-# tiles whose free pairs take two halves each
+# tiles, all of them single halves on 74 pairs; then whole tiles, with single halves behind them, and a part-filled round of whole
+# tiles whose free pairs take two halves each.  (Whole tiles of least K and cut tiles: test_wide_schedule.py.)
 SHAPES = [(256, 512, 256), (256, 512, 200), (129, 257, 1024), (300, 700, 520), (1000, 2000, 640), (2304, 4352, 264), (5000, 9000, 328), (20000, 1100, 264)]
 KINDS = [("half", "half", "TN", 1.0, 0.0), ("half", "half", "NT", 1.0, 0.0), ("half", "float", "NT", 1 / 128, 0.0), ("half", "half", "TN", 0.5, 2.0),
          ("float", "float", "TN", 1.0, 0.0), ("float", "float", "NT", 1.0, 0.0)]
