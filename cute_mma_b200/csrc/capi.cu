@@ -548,10 +548,10 @@ int launch_gemm_bn(int m, int n, int k, const void* A, int ldA, const void* B, i
     if (int rc = round_counters(st, stream, &rounds)) return rc;
   // Bands of 16 tile rows otherwise: the z-curve's coordinates cost every role up to 1 us of divisions before its first tile
   // (8943 x 1591 x 506 NT half 27.1 -> 25.5, 1800 x 2448 x 260 NT 14.5 -> 13.4, 901 x 3318 x 275 and single tiles level).  Column by column
-  // where at most four K steps leave little but the stores, which then fill whole columns of C one after the other: us on the
-  // z-curve / bands of 16 / columns 5646 x 23374 x 122 half 95 / 118 / 81, 25611 x 4507 x 73 98 / 109 / 84, 12000 x 12000 x 64 half to float
-  // 106 / 115 / 107, 8192 x 8192 x 128 50 / 36 / 36.
-  const bool stores_only = k2 == 0 && (k + T2::kBK - 1) / T2::kBK <= 4;
+  // where at most four K steps leave little but storing a C that does not fit L2: whole columns of C then fill one after the other.
+  // us on the z-curve / bands of 16 / columns 5646 x 23374 x 122 half 95 / 118 / 81, 25611 x 4507 x 73 98 / 109 / 84, 12000 x 12000 x 64 half
+  // to float 106 / 115 / 107; not for few columns of tiles, 25600 x 512 x 121 14.2 / 11.5 / 13.7, 43656 x 1680 x 96 TF32 - / 61 / 67.
+  const bool stores_only = k2 == 0 && (k + T2::kBK - 1) / T2::kBK <= 4 && n >= 4096 && static_cast<long long>(m) * n * static_cast<long long>(sizeof(TOut)) > 3ll * st->l2_bytes / 2;
   const int raster = opt(kOptRaster) >= 0 ? opt(kOptRaster) : big ? 8 : stores_only ? (m + 2 * T2::kBM - 1) / (2 * T2::kBM) : 16;
   // With the bands, the band's panel of A is what later waves read again and B streams past once per band:
   // A is loaded evict-last, B evict-first.  Same shape: DRAM reads 26.2 -> 17.6 GB per launch, 23.9 -> 22.4 ms.
