@@ -46,7 +46,8 @@ inline bool small_wins(int m, int n, int steps, bool whole_k, long long sms) {
 // products are 3 % slower (216 shapes) up to 48 K steps, or 320 in a row, and beyond that (71) as the NT ones: 1600 x 3840 x 4928
 // half to float 56 / 60, 3583 x 5376 x 448 TF32 39 / 42, 5117 x 9734 x 3328 269 / 274 (0.97 in long runs), 1600 x 12608 x 7680 327 / 313 (0.93).
 // In between the two are level where whole wide tiles fill their rounds to five sixths (and 48 steps each): 2048 x 4096 x 3648 55.7 / 55.9,
-// 4096 x 2048 x 4096 behind the rotation of the weight (A_RW) 77.0 / 75.6.
+// 4096 x 2048 x 4096 behind the rotation of the weight (A_RW) 77.0 / 75.6.  Two columns of tiles are one wide one, which reads A once
+// for both: 0.96 over 16 shapes, 20480 x 331 x 6784 115 / 105, 21888 x 424 x 6272 121 / 111.
 // And there a last column of 256 without a neighbour, which reads all of A once more, costs more than its neighbours
 // save until they are eight or so: 49664 x 768 x 4672 NT 247 / 264, 12544 x 1792 x 2048 TF32 126 / 142, but 49664 x 1024 x 4672 343 / 337.
 inline bool wide_wins(int m, int n, int steps, bool nt, bool whole_lines, long long sms) {
@@ -54,7 +55,7 @@ inline bool wide_wins(int m, int n, int steps, bool nt, bool whole_lines, long l
   if (n <= 256 || rounds < 2 || rounds * steps < (nt ? 40 : 60) || (!nt && steps <= 8)) return false;
   if (!whole_lines) return true;
   const bool filled = tiles_n % 2 == 0 && 6 * tiles >= 5 * (rounds + rounds % 2) * pairs;
-  return (tiles_n % 2 == 0 || tiles_n >= 8) && (nt || (steps >= 48 && (filled || rounds * steps >= 320)));
+  return (tiles_n % 2 == 0 || tiles_n >= 8) && (nt || tiles_n == 2 || (steps >= 48 && (filled || rounds * steps >= 320)));
 }
 
 }  // namespace b200

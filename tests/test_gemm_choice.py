@@ -33,7 +33,7 @@ def test_small_or_pair(rules, m, n, steps, small, pair):
 
 # m, n, K steps, NT, rows on whole 128-byte lines, us on tiles of 256 x 256 / of 256 x 512
 @pytest.mark.parametrize("m,n,steps,nt,lines,pair,wide", [(12544, 1792, 64, 0, 1, 126, 142), (12544, 768, 64, 0, 1, 55, 62), (49664, 768, 73, 1, 1, 247, 264),
-                                                          (48000, 768, 12, 0, 1, 47, 52), (4096, 2048, 64, 0, 1, 77.0, 75.6), (1152, 6144, 86, 0, 1, 87, 92), (49664, 704, 73, 0, 1, 240, 266), (3583, 5376, 14, 0, 1, 39, 42),
+                                                          (48000, 768, 12, 0, 1, 47, 52), (4096, 2048, 64, 0, 1, 77.0, 75.6), (1152, 6144, 86, 0, 1, 87, 92), (20480, 331, 106, 0, 1, 115, 105), (21888, 424, 98, 0, 1, 121, 111), (49664, 704, 73, 0, 1, 240, 266), (3583, 5376, 14, 0, 1, 39, 42),
                                                           (13171, 10088, 4, 0, 1, 98, 138), (8192, 8192, 128, 0, 1, 864, 831), (1600, 12608, 120, 0, 1, 327, 313),
                                                           (11008, 3001, 64, 0, 1, 252, 219), (4096, 4096, 256, 1, 1, 471, 436), (4096, 4096, 128, 1, 1, 221, 209),
                                                           (49664, 1024, 73, 1, 1, 343, 337), (5952, 6336, 17, 0, 0, 102, 83), (15713, 1302, 12, 0, 0, 55, 47),
