@@ -11,10 +11,10 @@ inline long long tiles_128(int m, int n) { return ((static_cast<long long>(m) + 
 // As long as its 128 x 128 tiles do not outnumber the SMs, always (fixed cost per launch 5 us against 7 to 9 us, and 256 x
 // 256 tiles leave most SMs idle: 640 x 1280 x 1024 TF32 29 -> 10 us), and for n <= 128, of which a pair tile covers twice
 // the columns at least (65536 x 120 x 4096 half 100 against 128 us, 131072 x 64 x 512 31 against 40).  Above, the two are
-// compared by a model fitted to 550 random shapes of 149 to 1500 tiles: a K step of two tiles per SM costs 0.74 us for 128
-// columns and 0.6 of that for the 128 rows of P alone (a narrow tile loads and multiplies those all the same), a last wave of one tile
+// compared by a model fitted to 649 random shapes of 149 to 1500 tiles: a K step of two tiles per SM costs 0.74 us for 128
+// columns and half of that for the 128 rows of P alone (a narrow tile loads and multiplies those all the same), a last wave of one tile
 // per SM 0.24 and of more 0.48; a round of pair tiles 0.34 us per step on 74 pairs, either size; plus fixed costs.  What it
-// picks takes 1 % longer than the better of the two on average, at worst 31 % (23650 x 310 x 1485 NT half to float 50.0 us against
+// picks takes 0.9 % longer than the better of the two on average, at worst 31 % (23650 x 310 x 1485 NT half to float 50.0 us against
 // 38.1).  Counted by its columns alone a narrow tile lost up to 55 % (7016 x 272 x 2536 half 29.5 against 21.0, 33475 x 147 x 2919 67.8
 // against 47.9).  5936 x 776 x 5822 NT: 118 against 68 us; 2815 x 6280 x 163: 27 against 20; 11904 x 276 x 263 TF32: 9.9 against 15.7.
 // With K whole (the GEMMs of oft_two_pass, n the rows of X) the model decides in the first range too, where a K step of an SM's only
@@ -26,10 +26,10 @@ inline bool small_wins(int m, int n, int steps, bool whole_k, long long sms) {
   const long long t256 = ((static_cast<long long>(m) + 255) / 256) * ((static_cast<long long>(n) + 255) / 256);
   const long long waves = t128 / (2 * sms), rest = t128 % (2 * sms);
   const int tiles_n = (n + 127) / 128;
-  const double step = (0.6 + 0.4 * ((n + tiles_n - 1) / tiles_n) / 128.0) * steps;  // K steps of 128 columns
+  const double step = (0.5 + 0.5 * ((n + tiles_n - 1) / tiles_n) / 128.0) * steps;  // K steps of 128 columns
   const double small = t128 <= sms ? 6.0 + 0.4 * step
-                                   : 6.0 + step * (0.74 * waves + (rest == 0 ? 0.0 : rest <= sms ? 0.24 : 0.48)) + 1.4 * (waves + (rest > 0));
-  const double pair = 8.0 + static_cast<double>((t256 + pairs - 1) / pairs) * (0.34 * steps + 1.4);
+                                   : 6.0 + step * (0.74 * waves + (rest == 0 ? 0.0 : rest <= sms ? 0.24 : 0.48)) + 1.8 * (waves + (rest > 0));
+  const double pair = 8.0 + static_cast<double>((t256 + pairs - 1) / pairs) * (0.34 * steps + 1.7);
   return small < pair;
 }
 
