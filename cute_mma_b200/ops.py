@@ -138,7 +138,11 @@ def oft_tn(m, n, k, A, ldA, B, ldB, R, ldR, C, ldC, stream=None, *, group_size=N
     group_size defaults to n (one block-diagonal R for all of N)."""
     lib = lib or load_library()
     gs = n if group_size is None else group_size
-    rc = getattr(lib, "direct_b200_oft_tn_f16", _not_taken)(m, n, k, gs, reconn_sz, A, ldA, B, ldB, R, ldR, C, ldC, stream)
+    try:
+        direct = lib.direct_b200_oft_tn_f16
+    except AttributeError:
+        direct = _not_taken
+    rc = direct(m, n, k, gs, reconn_sz, A, ldA, B, ldB, R, ldR, C, ldC, stream)
     if rc is None:
         rc = lib.b200_oft_tn_f16(m, n, k, gs, reconn_sz, _ptr(A), ldA, _ptr(B), ldB, _ptr(R), ldR, _ptr(C), ldC, _stream(stream))
     if rc != OK:
@@ -151,7 +155,11 @@ def oft_tn_two_pass(m, n, k, A, ldA, B, ldB, R, ldR, C, ldC, stream=None, *, gro
     header)."""
     lib = lib or load_library()
     gs = n if group_size is None else group_size
-    rc = getattr(lib, "direct_b200_oft_tn_f16_two_pass", _not_taken)(m, n, k, gs, reconn_sz, A, ldA, B, ldB, R, ldR, C, ldC, stream)
+    try:
+        direct = lib.direct_b200_oft_tn_f16_two_pass
+    except AttributeError:
+        direct = _not_taken
+    rc = direct(m, n, k, gs, reconn_sz, A, ldA, B, ldB, R, ldR, C, ldC, stream)
     if rc is None:
         rc = lib.b200_oft_tn_f16_two_pass(m, n, k, gs, reconn_sz, _ptr(A), ldA, _ptr(B), ldB, _ptr(R), ldR, _ptr(C), ldC, _stream(stream))
     if rc != OK:
@@ -280,7 +288,11 @@ def oft_tn_a_rw(m, n, k, A, ldA, B, ldB, R, ldR, C, ldC, stream=None, *, group_s
     """Same product as oft_tn computed as X . (R . W): weight transform, then one plain GEMM."""
     lib = lib or load_library()
     gs = n if group_size is None else group_size
-    rc = getattr(lib, "direct_b200_oft_tn_f16_a_rw", _not_taken)(m, n, k, gs, reconn_sz, A, ldA, B, ldB, R, ldR, C, ldC, stream)
+    try:
+        direct = lib.direct_b200_oft_tn_f16_a_rw
+    except AttributeError:
+        direct = _not_taken
+    rc = direct(m, n, k, gs, reconn_sz, A, ldA, B, ldB, R, ldR, C, ldC, stream)
     if rc is None:
         rc = lib.b200_oft_tn_f16_a_rw(m, n, k, gs, reconn_sz, _ptr(A), ldA, _ptr(B), ldB, _ptr(R), ldR, _ptr(C), ldC, _stream(stream))
     if rc != OK:
@@ -297,7 +309,11 @@ def oft_tn_host(m, n, k, A, ldA, B, ldB, R, ldR, C, ldC, *, group_size=None, rec
 def gemm_tn(m, n, k, A, ldA, B, ldB, C, ldC, stream=None, *, dtype="half", lib=None) -> None:
     """C(i,j) = sum_l A[i*ldA+l] B[j*ldB+l], C column-major.  dtype 'half' or 'float' (TF32)."""
     lib = lib or load_library()
-    rc = getattr(lib, "direct_b200_gemm_tn_f16" if dtype == "half" else "direct_b200_gemm_tn_tf32", _not_taken)(m, n, k, A, ldA, B, ldB, C, ldC, stream)
+    try:
+        direct = lib.direct_b200_gemm_tn_f16 if dtype == "half" else lib.direct_b200_gemm_tn_tf32
+    except AttributeError:
+        direct = _not_taken
+    rc = direct(m, n, k, A, ldA, B, ldB, C, ldC, stream)
     if rc is None:
         rc = (lib.b200_gemm_tn_f16 if dtype == "half" else lib.b200_gemm_tn_tf32)(m, n, k, _ptr(A), ldA, _ptr(B), ldB, _ptr(C), ldC, _stream(stream))
     if rc != OK:
@@ -307,7 +323,11 @@ def gemm_tn(m, n, k, A, ldA, B, ldB, C, ldC, stream=None, *, dtype="half", lib=N
 def gemm_nt(m, n, k, A, ldA, B, ldB, C, ldC, stream=None, *, dtype="half", lib=None) -> None:
     """C(i,j) = sum_l A[i+l*ldA] B[j+l*ldB], C column-major."""
     lib = lib or load_library()
-    rc = getattr(lib, "direct_b200_gemm_nt_f16" if dtype == "half" else "direct_b200_gemm_nt_tf32", _not_taken)(m, n, k, A, ldA, B, ldB, C, ldC, stream)
+    try:
+        direct = lib.direct_b200_gemm_nt_f16 if dtype == "half" else lib.direct_b200_gemm_nt_tf32
+    except AttributeError:
+        direct = _not_taken
+    rc = direct(m, n, k, A, ldA, B, ldB, C, ldC, stream)
     if rc is None:
         rc = (lib.b200_gemm_nt_f16 if dtype == "half" else lib.b200_gemm_nt_tf32)(m, n, k, _ptr(A), ldA, _ptr(B), ldB, _ptr(C), ldC, _stream(stream))
     if rc != OK:
@@ -327,7 +347,11 @@ def gemm_ex(transA, transB, m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, stream
     """C (column-major) = alpha * A.B^T + beta * C, half or float result from half operands, float from float (TF32)."""
     lib = lib or load_library()
     alpha, beta = float(alpha), float(beta)
-    rc = getattr(lib, "direct_b200_gemm_ex", _not_taken)(transA, transB, in_type, out_type, m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, stream)
+    try:
+        direct = lib.direct_b200_gemm_ex
+    except AttributeError:
+        direct = _not_taken
+    rc = direct(transA, transB, in_type, out_type, m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, stream)
     if rc is None:
         rc = lib.b200_gemm_ex(transA.encode(), transB.encode(), in_type, out_type, m, n, k, alpha, _ptr(A), ldA, _ptr(B), ldB, beta, _ptr(C), ldC,
                               _stream(stream))
